@@ -74,7 +74,7 @@ struct paratc_ctx {
     bool ztma32_ok = false;                    // that map is encoded (ncol even, nz supported)
     unsigned int* d_zt_err = nullptr;        // set by a TMA-fed kernel whose bounded wait ran out
     int sched_gen = 0;   // bumped whenever the Poisson schedule changes (captured graphs hold the old one)
-    double* d_pfac = nullptr;   // pivots of the spectral y systems (1/vecm, then arr), computed once
+    double* d_pfac = nullptr;   // pivots of the spectral y systems, computed once (k_pois_factors)
     DCoef* d_coef = nullptr;
     DDiag* d_diag = nullptr;
     DDiag* d_diag2 = nullptr;
@@ -389,7 +389,6 @@ void enqueue_substep32(paratc_ctx* ctx, int ns, int stop) {
     }
     ctx->launches += 1;
     if (stop == 1) return;
-    if (ctx->prm.scalar_on) { PROF(PK_HELM_SC); launch_helm_scalar(st, ctx->kc, ctx->d_coef, ctx->f32, ctx->d_hfac); ctx->launches++; }
     { PROF(PK_HELM); launch_helm(st, ctx->kc, ctx->d_coef, ctx->f32, ctx->d_duy_ym, ctx->d_uy_ym, ctx->d_hfac); }
     ctx->launches += 1;
     if (stop == 2) return;
@@ -421,7 +420,6 @@ void enqueue_substep(paratc_ctx* ctx, int ns, int stop = 5) {
     }
     ctx->launches += 1;
     if (stop == 1) return;
-    if (ctx->prm.scalar_on) { PROF(PK_HELM_SC); launch_helm_scalar(st, ctx->kc, ctx->d_coef, ctx->f, ctx->d_hfac); ctx->launches++; }
     { PROF(PK_HELM); launch_helm(st, ctx->kc, ctx->d_coef, ctx->f, ctx->d_duy_ym, ctx->d_uy_ym, ctx->d_hfac); }
     ctx->launches += 1;
     if (stop == 2) return;
@@ -713,8 +711,8 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
     kc.flow_type = prm->flow_type; kc.scalar_on = prm->scalar_on; kc.is_ux_const = prm->is_ux_const; kc.icfl = prm->icfl;
     cudaDeviceGetAttribute(&kc.nsm, cudaDevAttrMultiProcessorCount, ctx->dev);
     {
-        // PARATC_YSOLVER=staged|streaming pins the variant of the y-solve
-        // kernels (both are exact; the choice is normally made by size)
+        // PARATC_YSOLVER=staged|streaming sets the y bit of the schedule
+        // number; every grid takes the same y-solve kernel
         const char* e = std::getenv("PARATC_YSOLVER");
         kc.solver_sel = !e ? 0 : (std::strcmp(e, "staged") == 0 ? 1 : (std::strcmp(e, "streaming") == 0 ? 2 : 0));
     }
@@ -756,7 +754,7 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
         (rc = dalloc(ctx, &ctx->d_diag, 1)) || (rc = dalloc(ctx, &ctx->d_diag2, 1)) || (rc = dalloc(ctx, &ctx->d_scal, 16)) ||
         (rc = dalloc(ctx, &ctx->d_counter, 16)) ||
         (rc = dalloc(ctx, &ctx->d_hfac, helm_fac_doubles(ctx->ny))) ||
-        (rc = dalloc(ctx, &ctx->d_pfac, (size_t)2 * ctx->M1 * ctx->nz * ctx->ny)) ||
+        (rc = dalloc(ctx, &ctx->d_pfac, pois_fac_doubles(kc))) ||
         (rc = dalloc(ctx, &ctx->d_stats, (size_t)ctx->nyp * 40 + 1)) ||
         (rc = dalloc(ctx, &ctx->d_stats_part, stats_part_doubles(kc))) ||
         (rc = dalloc(ctx, &ctx->d_zt_err, 1))) {
@@ -1121,7 +1119,8 @@ int paratc_poisson(paratc_ctx* ctx, const double* src, double* phi) {
 
 // Poisson schedules: 2*s + (y-1), s 0 fused y-plane transforms, 1 separate
 // compile-time-length x / z transforms, 2 generic mixed-radix transforms, 3
-// as 1 with TMA-fed z transforms; y 1 staged, 2 streaming spectral y-solve
+// as 1 with TMA-fed z transforms; y, once the kind of the y-solve, selects
+// nothing (one kernel serves every grid) and is only handed back
 static bool sched_supported(const paratc_ctx* ctx, int choice) {
     if (choice < 0 || choice >= PARATC_SCHED_NCHOICES) return false;
     const int sc = choice / 2;
@@ -1215,6 +1214,7 @@ int paratc_autotune(paratc_ctx* ctx, int nrep, int* choice, double* times_ms) {
             if (!sched_supported(ctx, c)) continue;
             const bool f32 = ctx->prec == PARATC_PREC_FP32;
             if (f32 && c / 2 == 2) continue;  // the generic transforms have no float2 form
+            if (c % 2) continue;  // the y bit selects nothing: timed with its even neighbour
             sched_apply(ctx, c);
             // the step's form of the solve: divergence source, transforms,
             // y-solve, inverse into phi with its Neumann ghosts (state
@@ -1240,6 +1240,7 @@ int paratc_autotune(paratc_ctx* ctx, int nrep, int* choice, double* times_ms) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc != PARATC_OK) return rc;
+    for (int c = 1; c < PARATC_SCHED_NCHOICES; c += 2) tbest[c] = tbest[c - 1];
     int best = -1;
     for (int c = 0; c < PARATC_SCHED_NCHOICES; c++) {
         if (times_ms) times_ms[c] = tbest[c];
@@ -2065,8 +2066,8 @@ int grp_build(paratc_batch* b) {
     for (int ns = 1; ns <= maxiad && ok; ns++) {
         std::map<K4, GrpAcc<RhsArgs<double>>> rhs64;
         std::map<int, GrpAcc<RhsArgs<float>>> rhs32;
-        std::map<int, GrpAcc<HelmArgs<double>>> hs64, h64;
-        std::map<int, GrpAcc<HelmArgs<float>>> hs32, h32;
+        std::map<int, GrpAcc<HelmArgs<double>>> h64;
+        std::map<int, GrpAcc<HelmArgs<float>>> h32;
         std::map<int, GrpAcc<XfArgs<double, double2>>> xf64;
         std::map<int, GrpAcc<XfArgs<float, float2>>> xf32;
         std::map<int, GrpAcc<ZtArgs<double2>>> zt64;
@@ -2081,7 +2082,7 @@ int grp_build(paratc_batch* b) {
             if (c->hm.iadvance < ns) continue;
             const DConst& k = c->kc;
             const HostMetrics& h = c->hm;
-            const int M1 = c->nx / 2 + 1, kind = ys_kind(k);
+            const int M1 = c->nx / 2 + 1;
             const double gam = h.gam[ns - 1], the = h.the[ns - 1], alp = h.alp[ns - 1];
             if (c->prec == PARATC_PREC_FP32) {
                 float2* sp = spec32(c);
@@ -2089,18 +2090,15 @@ int grp_build(paratc_batch* b) {
                                                           the, alp, c->d_part, c->d_counter,
                                                           (int)rhs_member_grid(k, 1).x, 0},
                                        rhs_member_grid(k, 1));
-                if (c->prm.scalar_on)
-                    hs32[k.helm_var].add(k, HelmArgs<float>{k, c->d_coef, c->f32, nullptr, nullptr, c->d_hfac, 3},
-                                         helm_member_grid(k, 1), helm_smem(k));
-                h32[k.helm_var].add(k, HelmArgs<float>{k, c->d_coef, c->f32, c->d_duy_ym, c->d_uy_ym, c->d_hfac, 0},
-                                    helm_member_grid(k, 3), helm_smem(k));
+                h32[k.helm_var].add(k, HelmArgs<float>{k, c->d_coef, c->f32, c->d_duy_ym, c->d_uy_ym, c->d_hfac, 0, k.scalar_on ? 4 : 3},
+                                    helm_member_grid(k, k.scalar_on ? 4 : 3, 4), helm_smem(k, 4));
                 xf32[c->nx].add(k, XfArgs<float, float2>{k, c->dm, c->d_coef, c->f32.ux, c->f32.uy, c->f32.uz, sp,
                                                          c->d_twx, c->d_postx, c->d_part, c->d_counter + 1,
                                                          &c->d_coef->divmax_src},
                                 pfft_x_member_grid(k));
                 zt32[c->nz].add(k, ZtArgs<float2>{c->ny * M1, sp, c->d_twz}, pfft_z_member_grid(k));
-                ys32[kind].add(k, YsArgs<float2>{c->ny, M1, c->nz, c->dm.am2ph, sp, c->d_pfac},
-                               ys_member_grid(k, kind), ys_smem(k, kind));
+                ys32[0].add(k, YsArgs<float2>{c->ny, M1, c->nz, c->dm.am2ph, c->dm.ap2ph, sp, c->d_pfac},
+                            ys_member_grid(k, sizeof(float2)), ys_smem(k, sizeof(float2)));
                 xb32[c->nx].add(k, XbArgs<float2, float>{c->ny, c->nz, sp, c->d_phi32, c->d_twx, c->d_postx,
                                                          h.normfft},
                                 pfft_x_member_grid(k));
@@ -2113,18 +2111,15 @@ int grp_build(paratc_batch* b) {
                     k, RhsArgs<double>{k, c->dm, c->d_coef, c->f, c->d_uy_ym, c->d_duy_ym, gam, the, alp, c->d_part,
                                        c->d_counter, (int)rhs_member_grid(k, k.fp32_rhs).x, 0},
                     rhs_member_grid(k, k.fp32_rhs));
-                if (c->prm.scalar_on)
-                    hs64[k.helm_var].add(k, HelmArgs<double>{k, c->d_coef, c->f, nullptr, nullptr, c->d_hfac, 3},
-                                         helm_member_grid(k, 1), helm_smem(k));
-                h64[k.helm_var].add(k, HelmArgs<double>{k, c->d_coef, c->f, c->d_duy_ym, c->d_uy_ym, c->d_hfac, 0},
-                                    helm_member_grid(k, 3), helm_smem(k));
+                h64[k.helm_var].add(k, HelmArgs<double>{k, c->d_coef, c->f, c->d_duy_ym, c->d_uy_ym, c->d_hfac, 0, k.scalar_on ? 4 : 3},
+                                    helm_member_grid(k, k.scalar_on ? 4 : 3, 8), helm_smem(k, 8));
                 xf64[c->nx].add(k, XfArgs<double, double2>{k, c->dm, c->d_coef, c->f.ux, c->f.uy, c->f.uz, sp,
                                                            c->d_twx, c->d_postx, c->d_part, c->d_counter + 1,
                                                            &c->d_coef->divmax_src},
                                 pfft_x_member_grid(k));
                 zt64[c->nz].add(k, ZtArgs<double2>{c->ny * M1, sp, c->d_twz}, pfft_z_member_grid(k));
-                ys64[kind].add(k, YsArgs<double2>{c->ny, M1, c->nz, c->dm.am2ph, sp, c->d_pfac},
-                               ys_member_grid(k, kind), ys_smem(k, kind));
+                ys64[0].add(k, YsArgs<double2>{c->ny, M1, c->nz, c->dm.am2ph, c->dm.ap2ph, sp, c->d_pfac},
+                            ys_member_grid(k, sizeof(double2)), ys_smem(k, sizeof(double2)));
                 xb64[c->nx].add(k, XbArgs<double2, double>{c->ny, c->nz, sp, c->d_phi, c->d_twx, c->d_postx,
                                                            h.normfft},
                                 pfft_x_member_grid(k));
@@ -2148,8 +2143,8 @@ int grp_build(paratc_batch* b) {
         auto ztb = [](cudaStream_t st, int nz, const DConst&, auto tab, int nblk, size_t) {
             launch_zt_grp(st, 1, nz, tab, nblk);
         };
-        auto ys = [](cudaStream_t st, int kind, const DConst&, auto tab, int nblk, size_t sm) {
-            launch_ys_grp(st, kind, tab, nblk, sm);
+        auto ys = [](cudaStream_t st, int, const DConst&, auto tab, int nblk, size_t sm) {
+            launch_ys_grp(st, tab, nblk, sm);
         };
         auto xb = [](cudaStream_t st, int nx, const DConst&, auto tab, int nblk, size_t) { launch_xb_grp(st, nx, tab, nblk); };
         auto pj = [](cudaStream_t st, int, const DConst&, auto tab, int nblk, size_t) { launch_project_grp(st, tab, nblk); };
@@ -2158,7 +2153,6 @@ int grp_build(paratc_batch* b) {
         grp_balance_rhs(rhs64);
         grp_balance_rhs(rhs32);
         ok = ok && grp_emit(P, rhs64, L, rhs) && grp_emit(P, rhs32, L, rhs);
-        ok = ok && grp_emit(P, hs64, L, helm) && grp_emit(P, hs32, L, helm);
         ok = ok && grp_emit(P, h64, L, helm) && grp_emit(P, h32, L, helm);
         ok = ok && grp_emit(P, xf64, L, xf) && grp_emit(P, xf32, L, xf);
         ok = ok && grp_emit(P, zt64, L, ztf) && grp_emit(P, zt32, L, ztf);

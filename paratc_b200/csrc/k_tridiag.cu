@@ -14,10 +14,11 @@
 // Poisson systems, per context).  So the Thomas pivots are computed apart
 // from the solves, and a solve is a chain of multiply-adds per column with
 // its loads issued ahead: k_helm (pivots per step, k_helm_factors) and
-// k_ys_staged / k_ys_global (pivots per context, k_pois_factors).  The
+// k_ys_pair (pivots per context, k_pois_factors).  The
 // partitioned reduced-system solver (part_eliminate / part_reduced /
 // k_ysolve) computes its pivots in place; the allocation-free Poisson entry
 // point uses it because it has no room to keep pivots between calls.
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -148,186 +149,232 @@ struct PoisDiag {
 // Helmholtz: comp 0 ux (clcU1Hat), 1 uy (clcU2Hat), 2 uz (clcU3Hat),
 // 3 scalar (clcScalar); u(jc) += du(jc) with (I - beta*Lyy) du = Rhs
 // (src/m_TScheme.f90:365-506).  The matrices depend on the row only, so
-// their Thomas pivots (InverseTridiagonal, src/m_Tools.f90:224-251) are
-// computed once per step by k_helm_factors: for matrix (ns, type) and row jc,
-// A = a(jc), RV = 1/vecm(jc), AR = arr(jc), evaluated in the reference's
-// order without contraction.  A warp then sweeps 32 adjacent columns (i)
-// straight from memory: rows come in chunks of HY_U held in a three-chunk
-// register ring, so two chunks are in flight while one is on the dependent
-// chain.  The forward sweep writes f(jc) back over Rhs (it stays in L2 for
-// the backward sweep), the backward sweep adds the solution to u.
+// their pivots are computed once per step by k_helm_factors.  Every column is
+// eliminated from both walls at once, as in the spectral solve below: rows
+// 1 .. h = ny/2 upwards, rows ny .. h+1 downwards, and for row j of either
+// half the table holds r = 1 / pivot, MP = r times the coupling to the row
+// swept before, MN = r times the coupling to the row after, so that a row's
+// link of the chain is one FMA:
+//   F(j) = r (Rhs + add) - MP F(before),   x(j) = F(j) - MN x(after).
+// A work item is 32 adjacent columns of one component; a CTA is two warps,
+// one per wall, and walks items with a stride of its grid.  A warp's half of
+// the right-hand sides sits in its part of shared memory in sweep order
+// (copied there with cp.async; F replaces it row by row, so no forward-swept
+// value goes through memory), the sweep back reads u one chunk ahead, writes
+// u + x, and copies the next item's rows into the slots it has read.  The
+// columns are numbered through the planes (k nx + i), so that no lane idles
+// on a narrow or ragged nx.
 // uy and the scalar also get the ghost values that
 // SetBC_and_UpdateHaloForPrSrc / _scalar give them.
 // ---------------------------------------------------------------------------
 namespace {
-// rows per chunk (three chunks in registers, two in flight): 8, or 4 in the
-// tuner's second variant (DConst::helm_var = 1); twice that for float storage
-constexpr int HY_U = 8;
+constexpr int HY_U = 8;  // rows a sweep reads ahead of its chain; 4 in the tuner's second variant
 constexpr int HELM_NVAR = 2;
 __host__ __device__ inline int helm_stride(int ny) { return 3 * (ny + 2); }
+// shared memory of one wall's half of an item, hm rows: the columns, (r, MP)
+// pairs, MN
+__host__ __device__ inline int helm_half(int hm, int vsize, int wsize) {
+    const int b = hm * 32 * vsize + 3 * ((hm + 1) & ~1) * wsize;
+    return (b + 127) & ~127;
+}
+template <class W>
+struct W2;
+template <>
+struct W2<double> {
+    using T = double2;
+};
+template <>
+struct W2<float> {
+    using T = float2;
+};
 }  // namespace
 
-// thread = column i = 128*blockIdx.x + 32*threadIdx.y + lane at z index
-// blockIdx.y, component comp0 + blockIdx.z: the four warps of a CTA read
-// one contiguous 1 KB stretch of a row together.  The pivots sit in shared
-// memory; rows are addressed by pointer steps; the wall rows need no case of
-// their own in the sweeps (a(1) = 0, arr(ny+1) = 0, and clcU2Hat's row-1
-// value is substituted before the sweep and its result after it).
-// G: the block this CTA works as (OwnGrid, or SubGrid in a grouped launch).
-// Z4: the grouped launch's CTA shape, 32 columns of 4 z planes (one per
-// warp), so that a narrow member (nx < 128) leaves no warp idle.
-// W: the sweeps' arithmetic, double (FP64 in every form), or float for the
-// FP32 storage form's third launch shape, whose rows are stored in float
-// anyway: widening each value to FP64 and rounding it back put conversions
-// and FP64 latencies on every row of the chain
-template <class V, int HU, bool Z4 = false, class W = double, class G>
+// 16-byte copy that bypasses registers
+__device__ __forceinline__ void cpa16(void* sdst, const void* gsrc) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
+}
+
+// V: storage of the fields.  W: the sweeps' arithmetic, double (FP64 in every
+// form), or float for the FP32 storage form's third launch shape, whose rows
+// are stored in float anyway.  G: the block this CTA works as (OwnGrid, or
+// SubGrid in a grouped launch).
+template <class V, int U, class W, class G>
 __device__ __forceinline__ void helm_body(const G& grid, const DConst& cst, const DCoef* __restrict__ coef, int comp0,
-                                          const FieldSet<V>& fl, const double* __restrict__ duy_ym,
+                                          int ncomp, const FieldSet<V>& fl, const double* __restrict__ duy_ym,
                                           const double* __restrict__ uy_ym, const double* __restrict__ facs) {
-    extern __shared__ double shf[];
-    const int nx = cst.nx, ny = cst.ny;
-    const int comp = comp0 + (int)grid.z();
-    const int t = comp == 1 ? 1 : (comp == 3 ? 2 : 0);
+    using WP = typename W2<W>::T;
+    constexpr int VL = 16 / (int)sizeof(V), LPR = 32 / VL, RPW = 32 / LPR;  // a copy's columns, lanes per row, rows per pass
+    extern __shared__ __align__(128) unsigned char hm_raw[];
+    __shared__ WP xch[2][2][32];  // [item parity][wall][lane]: the last row's F and MN
+    const int nx = cst.nx, ny = cst.ny, nz = cst.nz;
+    const int end = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = ny >> 1, nt = end ? ny - h : h, hm = ny - h;
+    unsigned char* my = hm_raw + (size_t)end * helm_half(hm, sizeof(V), sizeof(W));
+    V* const sd = reinterpret_cast<V*>(my);
+    WP* const srp = reinterpret_cast<WP*>(my + (size_t)hm * 32 * sizeof(V));
+    W* const smn = reinterpret_cast<W*>(srp + ((hm + 1) & ~1));
+    const int dj = end ? -1 : 1, jw = end ? ny : 1;  // row i of the sweep is row jw + dj i
+    const ptrdiff_t gstep = (ptrdiff_t)dj * nx;
+    const int ncols = nx * nz, nct = (ncols + 31) / 32, nitems = nct * ncomp;
+    const int stride = (int)grid.gx();
+    const size_t pl = (size_t)cst.nyt * nx;
+    auto rhs_of = [&](int comp) { return comp == 0 ? fl.rx : comp == 1 ? fl.ry : comp == 2 ? fl.rz : fl.rc; };
+    auto u_of = [&](int comp) { return comp == 0 ? fl.ux : comp == 1 ? fl.uy : comp == 2 ? fl.uz : fl.sc; };
+    // copies: lane = (row of a pass, VL adjacent columns)
+    const int lr = lane / LPR, lc = (lane % LPR) * VL;
+    V* const cdst = sd + lr * 32 + lc;
+    const V* csrc = nullptr;  // row lr of the item's columns lc ..
+    bool cval = false;
+    auto aim = [&](int item) {
+        const int c = item / nct, q = (item - c * nct) * 32 + lc;
+        cval = q < ncols;
+        const int k = q / nx;
+        csrc = rhs_of(comp0 + c) + (size_t)k * pl + (q - k * nx) + (size_t)jw * nx + lr * gstep;
+    };
+    auto copy_rows = [&](int i0, int n) {  // rows i0 .. i0 + n - 1, n <= U
+        const V* src = csrc + i0 * gstep;
+#pragma unroll
+        for (int u = 0; u < U; u += RPW) {
+            if (cval && u + lr < n) cpa16(cdst + (i0 + u) * 32, src);
+            src += RPW * gstep;
+        }
+    };
+    int item = (int)grid.x();
+    if (item < nitems) aim(item);
     pdl_wait();
-    pdl_trigger();
-    {
-        const double* F = facs + (size_t)((coef->ns - 1) * 3 + t) * helm_stride(ny);
-        const int tid = threadIdx.y * 32 + threadIdx.x;
-        W* shw = reinterpret_cast<W*>(shf);
-        for (int q = tid; q < helm_stride(ny); q += 128) shw[q] = (W)F[q];
-    }
-    __syncthreads();
-    const W* SA = reinterpret_cast<const W*>(shf);
-    const W* SR = SA + (ny + 2);
-    const W* SW = SA + 2 * (ny + 2);
-    const int i = Z4 ? (int)grid.x() * 32 + (int)threadIdx.x : (int)(grid.x() * 4 + threadIdx.y) * 32 + (int)threadIdx.x;
-    const int k = Z4 ? (int)grid.y() * 4 + (int)threadIdx.y : (int)grid.y();
-    if (i >= nx || (Z4 && k >= cst.nz)) return;
-    V* u;
-    V* rhs;
-    double add = 0.0;
-    if (comp == 0)      { u = fl.ux; rhs = fl.rx; add = coef->rhsx_add; }
-    else if (comp == 1) { u = fl.uy; rhs = fl.ry; }
-    else if (comp == 2) { u = fl.uz; rhs = fl.rz; }
-    else                { u = fl.sc; rhs = fl.rc; }
-    const size_t col = (size_t)k * cst.nyt * nx + i;
-    // the sweeps run in W (FP64 unless chosen otherwise): loads convert, stores round
-    const W addw = (W)add;
-    V* rc = rhs + col;
-    V* uc = u + col;
-    const int nch = (ny + HU - 1) / HU;
-
-    // forward sweep, rows 1..ny: f = ((r + add) - a f_prev) / vecm, written over Rhs
-    const double a0 = (comp == 1) ? duy_ym[(size_t)k * nx + i] : 0.0;
-    // the register ring holds rows in their storage type and widens them
-    // where they are used, so that the loads of later chunks stay in flight
-    V A[HU], B[HU], C[HU];
-    auto ldr = [&](V (&X)[HU], int cc) {
-        if (cc >= nch) return;
-        const V* b = rc + (size_t)(cc * HU + 1) * nx;
-        const int nr = ny - cc * HU;
-#pragma unroll
-        for (int q = 0; q < HU; q++) {
-            if (q < nr) X[q] = *b;
-            b += nx;
-        }
-    };
-    W fp = 0;
-    V* wp = rc + nx;
-    auto fwd = [&](const V (&X)[HU], int cc) {
-        if (cc >= nch) return;
-        const int nr = ny - cc * HU;
-        const W* sa = SA + cc * HU + 1;
-        const W* sr = SR + cc * HU + 1;
-#pragma unroll
-        for (int q = 0; q < HU; q++) {
-            if (q < nr) {
-                // clcU2Hat: the row-1 value is the wall increment (kept in FP64)
-                const W xq = (comp == 1 && cc == 0 && q == 0) ? (W)a0 : (W)X[q];
-                const W f = ((xq + addw) - sa[q] * fp) * sr[q];
-                *wp = (V)f;
-                fp = f;  // the chain stays in W (no conversion on the dependent path)
+    if (item < nitems)
+        for (int i0 = 0; i0 < nt; i0 += U) copy_rows(i0, min(U, nt - i0));
+    const int nb = nt - 1, nf = nt / U * U, nbf = nb / U * U;
+    int type = -1;
+    for (int it = 0; item < nitems; item += stride, it++) {
+        const int next = item + stride;
+        if (next >= nitems) pdl_trigger();
+        const int comp = comp0 + item / nct;
+        const int t = comp == 1 ? 1 : (comp == 3 ? 2 : 0);
+        if (t != type) {  // this matrix's table, in sweep order
+            type = t;
+            const double* F = facs + (size_t)((coef->ns - 1) * 3 + t) * helm_stride(ny);
+            for (int i = lane; i < nt; i += 32) {
+                const int j = jw + dj * i;
+                WP p;
+                p.x = (W)F[(ny + 2) + j];
+                p.y = (W)F[j];
+                srp[i] = p;
+                smn[i] = (W)F[2 * (ny + 2) + j];
             }
-            wp += nx;
         }
-    };
-    ldr(A, 0);
-    ldr(B, 1);
-    ldr(C, 2);
-    for (int c = 0; c < nch; c += 3) {
-        fwd(A, c);
-        ldr(A, c + 3);
-        fwd(B, c + 1);
-        ldr(B, c + 4);
-        fwd(C, c + 2);
-        ldr(C, c + 5);
-    }
-    // backward sweep, rows ny..1: x = f - arr(j+1) x(j+1), u += x
-    V DA[HU], DB[HU], DC[HU], UA[HU], UB[HU], UC[HU];
-    auto ldb = [&](V (&D)[HU], V (&U)[HU], int cc) {
-        if (cc >= nch) return;
-        const size_t off = (size_t)(ny - cc * HU) * nx;
-        const V* bd = rc + off;
-        const V* bu = uc + off;
-        const int nr = ny - cc * HU;
+        const int q = (item % nct) * 32 + lane, k = q / nx;
+        const bool valid = q < ncols;
+        const size_t col = (size_t)k * pl + (q - k * nx);
+        V* const uc = u_of(comp) + col;
+        const W add = comp == 0 ? (W)coef->rhsx_add : (W)0;
+        // clcU2Hat: the row-1 value is the wall increment (kept in FP64)
+        const bool v1 = comp == 1 && end == 0;
+        const W a0 = v1 && valid ? (W)duy_ym[q] : (W)0;
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncwarp();
+        V* const s = sd + lane;
+        W f = 0;
+        for (int i0 = 0; i0 < nf; i0 += U) {
+            W g[U], mm[U];
 #pragma unroll
-        for (int q = 0; q < HU; q++) {
-            if (q < nr) { D[q] = *bd; U[q] = *bu; }
-            bd -= nx;
-            bu -= nx;
-        }
-    };
-    W xn = 0, unew = 0, utop = 0;
-    V* up = uc + (size_t)ny * nx;
-    auto bwd = [&](const V (&D)[HU], const V (&U)[HU], int cc) {
-        if (cc >= nch) return;
-        const int nr = ny - cc * HU;
-        const W* sw = SW + ny + 1 - cc * HU;
-#pragma unroll
-        for (int q = 0; q < HU; q++) {
-            if (q < nr) {
-                const W x = (W)D[q] - sw[-q] * xn;
-                xn = x;
-                unew = (W)U[q] + x;
-                *up = (V)unew;
+            for (int u = 0; u < U; u++) {
+                const WP p = srp[i0 + u];
+                g[u] = ((W)s[(i0 + u) * 32] + add) * p.x;
+                mm[u] = p.y;
             }
-            up -= nx;
+            if (v1 && i0 == 0) g[0] = a0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                f = g[u] - mm[u] * f;
+                s[(i0 + u) * 32] = (V)f;
+            }
         }
-    };
-    ldb(DA, UA, 0);
-    ldb(DB, UB, 1);
-    ldb(DC, UC, 2);
-    for (int c = 0; c < nch; c += 3) {
-        bwd(DA, UA, c);
-        if (c == 0) utop = (W)DA[0] + (W)UA[0];  // u(ny): x(ny) = f(ny)
-        ldb(DA, UA, c + 3);
-        bwd(DB, UB, c + 1);
-        ldb(DB, UB, c + 4);
-        bwd(DC, UC, c + 2);
-        ldb(DC, UC, c + 5);
-    }
-    // wall rows: unew now holds u(1)
-    if (comp == 1) {
-        uc[nx] = (V)uy_ym[(size_t)k * nx + i];
-        uc[(size_t)(ny + 1) * nx] = (V)((cst.flow_type == 1) ? cst.uybc_yp : 0.0);
-    } else if (comp == 3) {
-        uc[0] = (V)(cst.sc_r1b * (double)unew + cst.sc_r2b);
-        uc[(size_t)(ny + 1) * nx] = (V)(cst.sc_r1t * (double)utop + cst.sc_r2t);
+        for (int i = nf; i < nt; i++) {
+            const WP p = srp[i];
+            f = (v1 && i == 0 ? a0 : ((W)s[i * 32] + add) * p.x) - p.y * f;
+            s[i * 32] = (V)f;
+        }
+        WP mine;
+        mine.x = f;
+        mine.y = smn[nb];
+        xch[it & 1][end][lane] = mine;
+        __syncthreads();
+        const WP o = xch[it & 1][end ^ 1][lane];
+        W x = (f - mine.y * o.x) / ((W)1 - mine.y * o.y);
+        // back to the wall: x(i) = F(i) - MN x(i+1), u += x
+        V* up = uc + (ptrdiff_t)(jw + dj * nb) * nx;
+        W un = 0;
+        if (valid) {
+            un = (W)*up + x;
+            *up = (V)un;
+        }
+        for (int i = nb - 1; i >= nbf; i--) {
+            x = (W)s[i * 32] - smn[i] * x;
+            up -= gstep;
+            if (valid) {
+                un = (W)*up + x;
+                *up = (V)un;
+            }
+        }
+        V un0[U], un1[U];  // u of the chunk at hand and the one after it, in storage type
+        auto ldu = [&](V (&X)[U], const V* p) {
+#pragma unroll
+            for (int u = U - 1; u >= 0; u--) {
+                p -= gstep;
+                if (valid) X[u] = *p;
+            }
+        };
+        if (nbf > 0) ldu(un0, up);
+        __syncwarp();
+        if (next < nitems) {
+            aim(next);
+            copy_rows(nbf, nt - nbf);
+        }
+        for (int i0 = nbf - U; i0 >= 0; i0 -= U) {
+            if (i0 > 0) ldu(un1, up - U * gstep);
+            W d[U], mm[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                d[u] = (W)s[(i0 + u) * 32];
+                mm[u] = smn[i0 + u];
+            }
+            __syncwarp();
+            if (next < nitems) copy_rows(i0, U);
+#pragma unroll
+            for (int u = U - 1; u >= 0; u--) {
+                x = d[u] - mm[u] * x;
+                up -= gstep;
+                un = (W)un0[u] + x;
+                if (valid) *up = (V)un;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) un0[u] = un1[u];
+        }
+        // the wall rows: un holds u(1) or u(ny)
+        if (comp == 1 && valid) {
+            if (end == 0) uc[nx] = (V)uy_ym[q];
+            else uc[(size_t)(ny + 1) * nx] = (V)((cst.flow_type == 1) ? cst.uybc_yp : 0.0);
+        } else if (comp == 3 && valid) {
+            if (end == 0) uc[0] = (V)(cst.sc_r1b * (double)un + cst.sc_r2b);
+            else uc[(size_t)(ny + 1) * nx] = (V)(cst.sc_r1t * (double)un + cst.sc_r2t);
+        }
     }
 }
 
-template <class V, int HU, class W = double>
-__global__ void __launch_bounds__(128, 4) k_helm(DConst cst, const DCoef* __restrict__ coef, int comp0, FieldSet<V> fl,
-                                              const double* __restrict__ duy_ym, const double* __restrict__ uy_ym,
-                                              const double* __restrict__ facs) {
-    helm_body<V, HU, false, W>(OwnGrid{}, cst, coef, comp0, fl, duy_ym, uy_ym, facs);
+template <class V, int U, class W = double>
+__global__ void __launch_bounds__(64, 8) k_helm(DConst cst, const DCoef* __restrict__ coef, int comp0, int ncomp,
+                                                FieldSet<V> fl, const double* __restrict__ duy_ym,
+                                                const double* __restrict__ uy_ym, const double* __restrict__ facs) {
+    helm_body<V, U, W>(OwnGrid{}, cst, coef, comp0, ncomp, fl, duy_ym, uy_ym, facs);
 }
 
-template <class V, int HU, class W = double>
-__global__ void __launch_bounds__(128, 4) k_helm_grp(const GrpTab<HelmArgs<V>>* __restrict__ t) {
+template <class V, int U, class W = double>
+__global__ void __launch_bounds__(64, 8) k_helm_grp(const GrpTab<HelmArgs<V>>* __restrict__ t) {
     SubGrid g;
     const HelmArgs<V>& a = t->e[grp_member(t, g)];
-    helm_body<V, HU, true, W>(g, a.c, a.coef, a.comp0, a.fl, a.duy_ym, a.uy_ym, a.fac);
+    helm_body<V, U, W>(g, a.c, a.coef, a.comp0, a.ncomp, a.fl, a.duy_ym, a.uy_ym, a.fac);
 }
 
 // ---------------------------------------------------------------------------
@@ -382,346 +429,265 @@ __global__ void __launch_bounds__(512) k_ysolve(DConst cst, DMetric m, double* _
 // ---------------------------------------------------------------------------
 // Spectral y-solve with the factors computed once.  The Poisson matrices
 // (am2ph, ac2ph + lambda_x(kx) + lambda_z(kz), ap2ph) depend on the mesh and
-// the wavenumbers only, so the pivots of InverseTridiagonal
-// (src/m_Tools.f90:224-251) are computed once per context: for complex
-// column q = kz*(nx/2+1) + kx and Fortran row jc, rv[(jc-1)*NQ + q] =
-// 1/vecm(jc) and ar[(jc-1)*NQ + q] = arr(jc) (two arrays, so that each sweep
-// reads only the one it needs) with vecm(1) = b(1), arr(jc) = c(jc-1)/vecm(jc-1),
-// vecm(jc) = b(jc) - a(jc)*arr(jc), evaluated in the reference's order
-// without contraction.  A solve is then the two sweeps
-//   f(1) = f(1)/vecm(1),  f(jc) = (f(jc) - a(jc) f(jc-1)) / vecm(jc),
-//   f(jc) = f(jc) - arr(jc+1) f(jc+1),
-// with no division left on the dependent chain (1/vecm is a multiply).
-// The kx = kz = 0 system has row 1 replaced by phi = 0 (b = 1, c = 0,
-// f = 0; src/m_Poisson.f90:399-404).
+// the wavenumbers only, so their pivots are computed once per context.  Every
+// system is eliminated from both walls at once: rows 1 .. h = ny/2 downwards
+// from the lower wall, rows ny .. h+1 from the upper one,
+//   lower:  x(j) = F(j) - c(j) r(j) x(j+1),  F(j) = r(j) (f(j) - a(j) F(j-1)),
+//           r(j) = 1 / (b(j) - a(j) c(j-1) r(j-1)),
+//   upper:  the same with a and c exchanged and the rows reversed,
+// so that the two dependent chains of a column are half as long as the one
+// of InverseTridiagonal (src/m_Tools.f90:224-251) and run side by side; the
+// two equations that meet at rows h, h+1 give both unknowns, and the sweeps
+// return to the walls.  Only r is kept: the multipliers a r and c r are one
+// multiply off the chain.  lambda_z is even in kz, so the columns kz and
+// nz - kz share their pivots: the table holds kz = 0 .. nz/2, blocks of YP_C
+// modes kx, [kz][block][row][YP_C] -- a quarter of one FP64 factor pair per
+// spectrum value.  The kx = kz = 0 system has row 1 replaced by phi = 0
+// (b = 1, c = 0, f = 0; src/m_Poisson.f90:399-404).
 // ---------------------------------------------------------------------------
-// dc_here: column 0 is the kx = kz = 0 system (false for a z-slab rank
-// whose modes start above kx = 0; m.wnx then starts at its first mode)
-__device__ __forceinline__ void pois_factors_body(int ny, int M1, int nz, const DMetric& m, double* __restrict__ rv,
-                                                  double* __restrict__ ar, bool dc_here) {
-    const int NQ = M1 * nz;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= NQ) return;
-    const int kz = q / M1, kx = q - kz * M1;
-    const double wx = m.wnx[kx], wz = m.wnz[kz];
-    const bool dc = dc_here && (q == 0);
-    double vecm = dc ? 1.0 : __dadd_rn(__dadd_rn(m.ac2ph[1], wx), wz);
-    rv[q] = 1.0 / vecm;
-    ar[q] = 0.0;
-    for (int jc = 2; jc <= ny; jc++) {
-        const double cp = (dc && jc == 2) ? 0.0 : m.ap2ph[jc - 1];
-        const double arr = cp / vecm;
-        const double b = __dadd_rn(__dadd_rn(m.ac2ph[jc], wx), wz);
-        vecm = __dsub_rn(b, __dmul_rn(m.am2ph[jc], arr));
-        rv[(size_t)(jc - 1) * NQ + q] = 1.0 / vecm;
-        ar[(size_t)(jc - 1) * NQ + q] = arr;
-    }
-}
-__global__ void k_pois_factors(int ny, int M1, int nz, DMetric m, double* __restrict__ rv, double* __restrict__ ar) {
-    pois_factors_body(ny, M1, nz, m, rv, ar, true);
-}
-__global__ void k_pois_factors_slab(int ny, int M1, int nz, DMetric m, double* __restrict__ rv, double* __restrict__ ar,
-                                    int dc_here) {
-    pois_factors_body(ny, M1, nz, m, rv, ar, dc_here != 0);
+namespace {
+constexpr int YP_C = 8;  // complex columns of one kz in a work item: 128 bytes of a spectrum row
+constexpr int YP_U = 8;  // rows a sweep reads ahead of its chain
+__host__ __device__ inline int yp_blocks(int M1) { return (M1 + YP_C - 1) / YP_C; }
+
+// esize-byte copy that bypasses registers (16: double2, 8: float2)
+template <int N>
+__device__ __forceinline__ void cpa(void* sdst, const void* gsrc) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
+    if constexpr (N == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
 }
 
-namespace {
-__device__ __forceinline__ void cpa16t(void* sdst, const void* gsrc) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
+// shared memory of one wall's half of an item, hm rows: the two planes' boxes
+// (with a float2 spectrum, whose rows are 64 bytes, the second box starts half
+// a bank cycle after the first, so that a warp's two half-rows fall into
+// different banks), the pivots, the two couplings
+__host__ __device__ inline int yp_box(int hm, int esize) {
+    const int b = hm * YP_C * esize;
+    return esize == 8 && b % 128 == 0 ? b + 64 : b;
 }
-__device__ __forceinline__ void cpa8t(void* sdst, const void* gsrc) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
+__host__ __device__ inline int yp_half(int hm, int esize) {
+    const int b = 2 * yp_box(hm, esize) + (hm * YP_C + 2 * ((hm + 1) & ~1)) * (int)sizeof(double);
+    return (b + 127) & ~127;
 }
-constexpr int YS_U = 8;  // rows loaded ahead of the dependent chain
 }  // namespace
 
-// Small grids (one wave): a one-warp CTA stages 16 complex columns of the
-// spectrum and their factors in shared memory with cp.async, then lane l
-// sweeps the real (l even) or imaginary (l odd) part of column l/2.  S: the
-// spectrum's storage (double2, or float2 in the FP32 storage form; the
-// sweeps run in double either way).
+// dc_here: column 0 is the kx = kz = 0 system (false for a z-slab rank
+// whose modes start above kx = 0; m.wnx then starts at its first mode)
+__global__ void k_pois_factors(int ny, int M1, int nz, DMetric m, double* __restrict__ fac, int dc_here) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= M1 * (nz / 2 + 1)) return;
+    const int kz = q / M1, kx = q - kz * M1;
+    const double wx = m.wnx[kx], wz = m.wnz[kz];
+    const bool dc = dc_here && q == 0;
+    double* r = fac + (size_t)(kz * yp_blocks(M1) + kx / YP_C) * ny * YP_C + kx % YP_C;
+    const int h = ny >> 1;
+    double vecm = dc ? 1.0 : __dadd_rn(__dadd_rn(m.ac2ph[1], wx), wz);
+    // a pivot of 0 makes both sweeps leave phi = 0 in the pinned row
+    r[0] = dc ? 0.0 : 1.0 / vecm;
+    for (int jc = 2; jc <= h; jc++) {
+        const double arr = ((dc && jc == 2) ? 0.0 : m.ap2ph[jc - 1]) / vecm;
+        const double b = __dadd_rn(__dadd_rn(m.ac2ph[jc], wx), wz);
+        vecm = __dsub_rn(b, __dmul_rn(m.am2ph[jc], arr));
+        r[(size_t)(jc - 1) * YP_C] = 1.0 / vecm;
+    }
+    vecm = __dadd_rn(__dadd_rn(m.ac2ph[ny], wx), wz);
+    r[(size_t)(ny - 1) * YP_C] = 1.0 / vecm;
+    for (int jc = ny - 1; jc > h; jc--) {
+        const double arr = m.am2ph[jc + 1] / vecm;
+        const double b = __dadd_rn(__dadd_rn(m.ac2ph[jc], wx), wz);
+        vecm = __dsub_rn(b, __dmul_rn(m.ap2ph[jc], arr));
+        r[(size_t)(jc - 1) * YP_C] = 1.0 / vecm;
+    }
+}
+
+// A work item is YP_C modes kx of the planes kz and nz - kz: 32 real columns
+// (lane = plane, mode, real or imaginary part).  A CTA is two warps, one per
+// wall, and walks items with a stride of its grid.  A warp's half of the
+// columns and their pivots sits in its own part of shared memory in the order
+// it sweeps them, copied there row by row with cp.async; while the sweep back
+// leaves a row (the solution goes straight to memory) the next item's row is
+// copied into the slot.  So a column crosses memory once each way, a row's
+// link of the chain is a single FMA, and the warps of an SM's CTAs keep
+// copies in flight all the time.
 template <class S, class G>
-__device__ __forceinline__ void ys_staged_body(const G& grid, int ny, int M1, int nz, const double* __restrict__ am2ph,
-                                               S* __restrict__ spec, const double* __restrict__ fac,
-                                               bool dc_here = true) {
+__device__ __forceinline__ void ys_pair_body(const G& grid, int ny, int M1, int nz, const double* __restrict__ am2ph,
+                                             const double* __restrict__ ap2ph, S* __restrict__ spec,
+                                             const double* __restrict__ fac) {
     using R = decltype(S::x);
-    extern __shared__ double2 sy[];
-    const int lane = threadIdx.x;
-    const int NQ = M1 * nz;
-    const int q0 = grid.x() * 16;
-    const int nv = min(16, NQ - q0);
-    S* sd = reinterpret_cast<S*>(sy);                          // [ny][16] spectrum
-    double* srv = reinterpret_cast<double*>(sy + ny * 16);     // [ny][16] 1/vecm
-    double* sar = srv + ny * 16;                               // [ny][16] arr
-    double* sa = sar + ny * 16;                                // am2ph[0..ny]
-    pdl_wait();
-    pdl_trigger();
-    // one 16-byte copy per lane and row: lanes 0-15 the spectrum of column
-    // q0+lane, lanes 16-23 two 1/vecm of columns q0+2(lane-16)+{0,1}, lanes
-    // 24-31 two arr (NQ is even, so the pairs are aligned and never split)
-    const int cq = lane & 15, half = lane >> 4;
-    const bool cval = cq < nv;
-    const int qq = q0 + (cval ? cq : 0);
-    const int kz = qq / M1, kx = qq - kz * M1;
-    S* scol = spec + (size_t)kz * ny * M1 + kx;
-    const char* gsrc;
-    char* sdst;
-    size_t gstride;
-    int sstride;
-    bool cvalid;
-    if (lane < 16) {
-        gsrc = reinterpret_cast<const char*>(scol);
-        gstride = (size_t)M1 * sizeof(S);
-        sdst = reinterpret_cast<char*>(sd + lane);
-        sstride = 16 * sizeof(S);
-        cvalid = cval;
-    } else {
-        const int pr = (lane & 7) * 2;
-        const double* base = fac + (lane < 24 ? (size_t)0 : (size_t)NQ * ny) + q0 + pr;
-        gsrc = reinterpret_cast<const char*>(base);
-        gstride = (size_t)NQ * sizeof(double);
-        sdst = reinterpret_cast<char*>((lane < 24 ? srv : sar) + pr);
-        sstride = 16 * sizeof(double);
-        cvalid = pr < nv;
+    constexpr int ES = (int)sizeof(S), ROW = YP_C * ES;  // bytes of a row of one plane
+    extern __shared__ __align__(128) unsigned char yp_raw[];
+    __shared__ double2 xch[2][2][32];  // [item parity][wall][lane]: the last row's F and its coupling
+    const int end = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = ny >> 1, nt = end ? ny - h : h, hm = ny - h;
+    const int box = yp_box(hm, ES);
+    unsigned char* my = yp_raw + (size_t)end * yp_half(hm, ES);
+    double* sr = reinterpret_cast<double*>(my + 2 * box);  // [hm][YP_C] pivots
+    double* cp = sr + (size_t)hm * YP_C;                   // couplings to the row before, to the row after
+    double* cn = cp + ((hm + 1) & ~1);
+    for (int i = lane; i < nt; i += 32) {
+        cp[i] = end ? ap2ph[ny - i] : am2ph[i + 1];
+        cn[i] = end ? am2ph[ny - i] : ap2ph[i + 1];
     }
-    if (cvalid) {
-        if (lane < 16 && sizeof(S) == 8)
-            for (int j = 0; j < ny; j++) cpa8t(sdst + (size_t)j * sstride, gsrc + (size_t)j * gstride);
-        else
-            for (int j = 0; j < ny; j++) cpa16t(sdst + (size_t)j * sstride, gsrc + (size_t)j * gstride);
-    }
-    for (int j = lane; j <= ny; j += 32) sa[j] = __ldg(&am2ph[j]);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    R* sdd = reinterpret_cast<R*>(sd);
-    const int cp = lane >> 1;  // complex column of this lane's real or imaginary part
-    const bool dc = dc_here && (q0 + cp) == 0;
-    double fp = 0.0;
-    for (int j0 = 0; j0 < ny; j0 += YS_U) {
-        double d[YS_U], rv[YS_U], a[YS_U];
+    const int nkb = yp_blocks(M1), nitems = (nz / 2 + 1) * nkb;
+    const int stride = (int)grid.gx();
+    const int dj = end ? -1 : 1, jw = end ? ny - 1 : 0;  // row i of the sweep is memory row jw + dj i
+    const ptrdiff_t gstep = (ptrdiff_t)dj * M1;
+    // copies: lane = (row of a pair, plane, mode)
+    const int lc = lane & 7, lz = (lane >> 3) & 1, lr = lane >> 4;
+    unsigned char* const cdst = my + lz * box + lr * ROW + lc * ES;
+    double* const fdst = sr + 2 * lane;
+    const S* csrc = nullptr;       // row lr of the next item's column
+    const double* fsrc = nullptr;  // pivots of row lane / 4
+    bool cval = false;
+    auto aim = [&](int item) {
+        const int kz = item / nkb, kx = (item - kz * nkb) * YP_C + lc, kp = lz ? (kz ? nz - kz : 0) : kz;
+        cval = item < nitems && kx < M1 && (lz == 0 || kp != kz);
+        csrc = spec + (size_t)kp * ny * M1 + kx + jw * M1 + lr * gstep;
+        fsrc = fac + ((size_t)item * ny + jw + dj * (lane >> 2)) * YP_C + 2 * (lane & 3);
+    };
+    auto copy_fac = [&](int i0, int n) {  // rows i0 .. i0 + n - 1, n <= 8
+        if ((lane >> 2) < n) cpa<16>(fdst + i0 * YP_C, fsrc + (ptrdiff_t)dj * i0 * YP_C);
+    };
+    auto copy_rows = [&](int i0, int n) {
+        const S* src = csrc + i0 * gstep;
+        unsigned char* dst = cdst + i0 * ROW;
 #pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 + u;
-            if (j < ny) {
-                d[u] = (double)sdd[j * 32 + lane];
-                rv[u] = srv[j * 16 + cp];
-                a[u] = sa[j + 1];
+        for (int u = 0; u < YP_U / 2; u++) {
+            if (cval && 2 * u + lr < n) cpa<ES>(dst + 2 * u * ROW, src);
+            src += 2 * gstep;
+        }
+    };
+    int item = (int)grid.x();
+    if (item < nitems) {
+        aim(item);
+        for (int i0 = 0; i0 < nt; i0 += YP_U) copy_fac(i0, nt - i0);
+    }
+    pdl_wait();  // the spectrum is written by the kernel before this one
+    if (item < nitems)
+        for (int i0 = 0; i0 < nt; i0 += YP_U) copy_rows(i0, nt - i0);
+    // sweeps: lane = (plane, mode, part)
+    const int pz = lane >> 4, col = (lane >> 1) & 7, part = lane & 1;
+    R* const sd = reinterpret_cast<R*>(my + pz * box) + col * 2 + part;
+    const double* const srl = sr + col;
+    const int nb = nt - 1, nf = nt & ~(YP_U - 1), nbf = nb & ~(YP_U - 1);
+    for (int it = 0; item < nitems; item += stride, it++) {
+        const int next = item + stride;
+        if (next >= nitems) pdl_trigger();
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncwarp();
+        // to the junction: F(i) = r (f - cp F(i-1)), kept in the row's slot
+        double f = 0.0;
+        for (int i0 = 0; i0 < nf; i0 += YP_U) {
+            double g[YP_U], mm[YP_U];
+#pragma unroll
+            for (int u = 0; u < YP_U; u++) {
+                const double r = srl[(i0 + u) * YP_C];
+                g[u] = (double)sd[(i0 + u) * 2 * YP_C] * r;
+                mm[u] = cp[i0 + u] * r;
+            }
+#pragma unroll
+            for (int u = 0; u < YP_U; u++) {
+                f = fma(-mm[u], f, g[u]);
+                sd[(i0 + u) * 2 * YP_C] = (R)f;
             }
         }
+        for (int i = nf; i < nt; i++) {
+            const double r = srl[i * YP_C];
+            f = fma(-(cp[i] * r), f, (double)sd[i * 2 * YP_C] * r);
+            sd[i * 2 * YP_C] = (R)f;
+        }
+        const double cu = cn[nb] * srl[nb * YP_C];
+        xch[it & 1][end][lane] = make_double2(f, cu);
+        __syncthreads();
+        const double2 o = xch[it & 1][end ^ 1][lane];
+        double x = (f - cu * o.x) / (1.0 - cu * o.y);
+        // back to the wall: x(i) = F(i) - cn r x(i+1), out to memory; the
+        // next item's rows follow into the slots just read
+        const int kz = item / nkb, kx = (item - kz * nkb) * YP_C + col, kp = pz ? (kz ? nz - kz : 0) : kz;
+        const bool valid = kx < M1 && (pz == 0 || kp != kz);
+        R* out = reinterpret_cast<R*>(spec + (size_t)kp * ny * M1 + kx + jw * M1 + nb * gstep) + part;
+        if (valid) *out = (R)x;
+        for (int i = nb - 1; i >= nbf; i--) {
+            x = fma(-(cn[i] * srl[i * YP_C]), x, (double)sd[i * 2 * YP_C]);
+            out -= 2 * gstep;
+            if (valid) *out = (R)x;
+        }
+        __syncwarp();
+        if (next < nitems) {
+            aim(next);
+            copy_fac(nbf, nt - nbf);
+            copy_rows(nbf, nt - nbf);
+        }
+        for (int i0 = nbf - YP_U; i0 >= 0; i0 -= YP_U) {
+            double d[YP_U], mm[YP_U];
 #pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 + u;
-            if (j < ny) {
-                const double f = (j == 0) ? (dc ? 0.0 : d[u]) * rv[u] : (d[u] - a[u] * fp) * rv[u];
-                sdd[j * 32 + lane] = (R)f;
-                fp = f;
+            for (int u = 0; u < YP_U; u++) {
+                d[u] = (double)sd[(i0 + u) * 2 * YP_C];
+                mm[u] = cn[i0 + u] * srl[(i0 + u) * YP_C];
+            }
+            __syncwarp();
+            if (next < nitems) {
+                copy_fac(i0, YP_U);
+                copy_rows(i0, YP_U);
+            }
+#pragma unroll
+            for (int u = YP_U - 1; u >= 0; u--) {
+                x = fma(-mm[u], x, d[u]);
+                out -= 2 * gstep;
+                if (valid) *out = (R)x;
             }
         }
     }
-    double xn = fp;
-    for (int j0 = ny - 2; j0 >= 0; j0 -= YS_U) {
-        double d[YS_U], ar[YS_U];
-#pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 - u;
-            if (j >= 0) {
-                d[u] = (double)sdd[j * 32 + lane];
-                ar[u] = sar[(j + 1) * 16 + cp];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 - u;
-            if (j >= 0) {
-                const double x = d[u] - ar[u] * xn;
-                sdd[j * 32 + lane] = (R)x;
-                xn = x;
-            }
-        }
-    }
-    __syncthreads();
-    if (cval)
-        for (int j = half; j < ny; j += 2) scol[(size_t)j * M1] = sd[j * 16 + cq];
 }
 
 template <class S>
-__global__ void __launch_bounds__(32) k_ys_staged(int ny, int M1, int nz, const double* __restrict__ am2ph,
-                                                  S* __restrict__ spec, const double* __restrict__ fac) {
-    ys_staged_body(OwnGrid{}, ny, M1, nz, am2ph, spec, fac);
+__global__ void __launch_bounds__(64, 8) k_ys_pair(int ny, int M1, int nz, const double* __restrict__ am2ph,
+                                                   const double* __restrict__ ap2ph, S* __restrict__ spec,
+                                                   const double* __restrict__ fac) {
+    ys_pair_body(OwnGrid{}, ny, M1, nz, am2ph, ap2ph, spec, fac);
 }
-
-// Large grids: one thread per real column straight from global memory, the
-// rows of a chunk loaded ahead of its chain, latency hidden by occupancy.
-// R: storage of the spectrum's real parts (double, or float in the FP32
-// storage form); the sweeps run in double either way
-template <class R, class G>
-__device__ __forceinline__ void ys_global_body(const G& grid, int ny, int M1, int nz, const double* __restrict__ am2ph,
-                                               R* __restrict__ specd, const double* __restrict__ fac,
-                                               bool dc_here = true) {
-    const int W = 2 * M1, NQ = M1 * nz;
-    const int g = grid.x() * blockDim.x + threadIdx.x;
-    pdl_wait();
-    pdl_trigger();
-    if (g >= W * nz) return;
-    const int kz = g / W, cr = g - kz * W, q = g >> 1;
-    R* col = specd + (size_t)kz * ny * W + cr;
-    const double* frv = fac + q;
-    const double* far = fac + (size_t)NQ * ny + q;
-    const bool dc = dc_here && (q == 0);
-    double fp = 0.0;
-    for (int j0 = 0; j0 < ny; j0 += YS_U) {
-        R d[YS_U];  // in the storage type: widened at use, so the loads stay in flight
-        double rv[YS_U], a[YS_U];
-#pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 + u;
-            if (j < ny) {
-                d[u] = col[(size_t)j * W];
-                rv[u] = __ldg(&frv[(size_t)j * NQ]);
-                a[u] = __ldg(&am2ph[j + 1]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 + u;
-            if (j < ny) {
-                const double du = (double)d[u];
-                const double f = (j == 0) ? (dc ? 0.0 : du) * rv[u] : (du - a[u] * fp) * rv[u];
-                col[(size_t)j * W] = (R)f;
-                fp = f;  // the chain stays FP64 (no conversion on the dependent path)
-            }
-        }
-    }
-    double xn = fp;
-    for (int j0 = ny - 2; j0 >= 0; j0 -= YS_U) {
-        R d[YS_U];
-        double ar[YS_U];
-#pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 - u;
-            if (j >= 0) {
-                d[u] = col[(size_t)j * W];
-                ar[u] = __ldg(&far[(size_t)(j + 1) * NQ]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < YS_U; u++) {
-            const int j = j0 - u;
-            if (j >= 0) {
-                const double x = (double)d[u] - ar[u] * xn;
-                col[(size_t)j * W] = (R)x;
-                xn = x;
-            }
-        }
-    }
-}
-
-template <class R>
-__global__ void __launch_bounds__(128) k_ys_global(int ny, int M1, int nz, const double* __restrict__ am2ph,
-                                                   R* __restrict__ specd, const double* __restrict__ fac) {
-    ys_global_body(OwnGrid{}, ny, M1, nz, am2ph, specd, fac);
-}
-
-// grouped: kind 0 staged (S the spectrum), 1 streaming (its real parts)
 template <class S>
-__global__ void __launch_bounds__(32) k_ys_staged_grp(const GrpTab<YsArgs<S>>* __restrict__ t) {
+__global__ void __launch_bounds__(64, 8) k_ys_pair_grp(const GrpTab<YsArgs<S>>* __restrict__ t) {
     SubGrid g;
     const YsArgs<S>& a = t->e[grp_member(t, g)];
-    ys_staged_body(g, a.ny, a.M1, a.nz, a.am2ph, a.spec, a.fac);
-}
-template <class S>
-__global__ void __launch_bounds__(128) k_ys_global_grp(const GrpTab<YsArgs<S>>* __restrict__ t) {
-    using R = decltype(S::x);
-    SubGrid g;
-    const YsArgs<S>& a = t->e[grp_member(t, g)];
-    ys_global_body(g, a.ny, a.M1, a.nz, a.am2ph, reinterpret_cast<R*>(a.spec), a.fac);
+    ys_pair_body(g, a.ny, a.M1, a.nz, a.am2ph, a.ap2ph, a.spec, a.fac);
 }
 
-void launch_pois_factors(cudaStream_t st, const DConst& c, const DMetric& m, double* fac) {
-    const int M1 = c.nx / 2 + 1, NQ = M1 * c.nz;
-    k_pois_factors<<<(NQ + 127) / 128, 128, 0, st>>>(c.ny, M1, c.nz, m, fac, fac + (size_t)NQ * c.ny);
+size_t pois_fac_doubles(const DConst& c) {
+    return (size_t)(c.nz / 2 + 1) * yp_blocks(c.nx / 2 + 1) * YP_C * c.ny;
+}
+void launch_pois_factors(cudaStream_t st, const DConst& c, const DMetric& m, double* fac, int dc_here) {
+    const int M1 = c.nx / 2 + 1, n = M1 * (c.nz / 2 + 1);
+    k_pois_factors<<<(n + 127) / 128, 128, 0, st>>>(c.ny, M1, c.nz, m, fac, dc_here);
 }
 
-// the same kernels for a z-slab rank's x-mode slab, whose column 0 is the
-// kx = kz = 0 system only on the rank holding kx = 0
-__global__ void __launch_bounds__(32) k_ys_staged_slab(int ny, int M1, int nz, const double* __restrict__ am2ph,
-                                                       double2* __restrict__ spec, const double* __restrict__ fac,
-                                                       int dc_here) {
-    ys_staged_body(OwnGrid{}, ny, M1, nz, am2ph, spec, fac, dc_here != 0);
+static size_t yp_smem(int ny, int esize) { return 2 * (size_t)yp_half(ny - ny / 2, esize); }
+size_t ys_smem(const DConst& c, int esize) { return yp_smem(c.ny, esize); }
+// a CTA per work item up to the CTAs the device holds at once (8 per SM by
+// registers, fewer by shared memory), which then walk the items
+dim3 ys_member_grid(const DConst& c, int esize) {
+    const int items = (c.nz / 2 + 1) * yp_blocks(c.nx / 2 + 1);
+    const int per_sm = (int)std::min<size_t>(8, (size_t)(224 * 1024) / (yp_smem(c.ny, esize) + 3072));
+    return dim3((unsigned)std::min(items, std::max(1, per_sm) * (c.nsm > 0 ? c.nsm : 148)));
 }
-__global__ void __launch_bounds__(128) k_ys_global_slab(int ny, int M1, int nz, const double* __restrict__ am2ph,
-                                                        double* __restrict__ specd, const double* __restrict__ fac,
-                                                        int dc_here) {
-    ys_global_body(OwnGrid{}, ny, M1, nz, am2ph, specd, fac, dc_here != 0);
-}
-void launch_pois_factors_slab(cudaStream_t st, const DConst& c, const DMetric& m, double* fac, int dc_here) {
-    const int M1 = c.nx / 2 + 1, NQ = M1 * c.nz;
-    k_pois_factors_slab<<<(NQ + 127) / 128, 128, 0, st>>>(c.ny, M1, c.nz, m, fac, fac + (size_t)NQ * c.ny, dc_here);
-}
-
-// the staged kernel's shared memory: the spectrum block (16 B per complex
-// value, whatever the storage, so that the factor arrays stay 16-byte
-// aligned), the two factor blocks and am2ph
-static size_t ys_staged_smem(int ny) { return (size_t)ny * 16 * 2 * sizeof(double2) + (size_t)(ny + 1) * sizeof(double); }
-
-// 0: the staged kernel (the grid fits one wave of it, or solver_sel = 1),
-// 1: the streaming one
-int ys_kind(const DConst& c) {
-    const int M1 = c.nx / 2 + 1, NQ = M1 * c.nz;
-    const size_t sm = ys_staged_smem(c.ny);
-    const int per_sm = sm > 0 ? (int)((220 * 1024) / sm) : 0;
-    const int ctas = (NQ + 15) / 16;
-    return (per_sm >= 1 && (c.solver_sel == 1 || (c.solver_sel == 0 && ctas <= per_sm * c.nsm))) ? 0 : 1;
-}
-dim3 ys_member_grid(const DConst& c, int kind) {
-    const int M1 = c.nx / 2 + 1, NQ = M1 * c.nz;
-    return kind == 0 ? dim3((NQ + 15) / 16) : dim3((2 * M1 * c.nz + 127) / 128);
-}
-size_t ys_smem(const DConst& c, int kind) { return kind == 0 ? ys_staged_smem(c.ny) : 0; }
 
 template <class S>
 static void ysolve_fac_t(cudaStream_t st, const DConst& c, const DMetric& m, S* spec, const double* fac) {
-    using R = decltype(S::x);
-    const int M1 = c.nx / 2 + 1;
-    const int kind = ys_kind(c);
-    if (kind == 0) {
-        launch_pdl(k_ys_staged<S>, ys_member_grid(c, 0), dim3(32), ys_smem(c, 0), st, c.ny, M1, c.nz, m.am2ph, spec,
-                   fac);
-    } else {
-        launch_pdl(k_ys_global<R>, ys_member_grid(c, 1), dim3(128), 0, st, c.ny, M1, c.nz, m.am2ph,
-                   reinterpret_cast<R*>(spec), fac);
-    }
-}
-
-template <class S>
-static void ys_grp_t(cudaStream_t st, int kind, const GrpTab<YsArgs<S>>* t, int nblk, size_t smem) {
-    if (kind == 0) launch_pdl(k_ys_staged_grp<S>, dim3((unsigned)nblk), dim3(32), smem, st, t);
-    else launch_pdl(k_ys_global_grp<S>, dim3((unsigned)nblk), dim3(128), 0, st, t);
-}
-void launch_ys_grp(cudaStream_t st, int kind, const GrpTab<YsArgs<double2>>* t, int nblk, size_t smem) {
-    ys_grp_t(st, kind, t, nblk, smem);
-}
-void launch_ys_grp(cudaStream_t st, int kind, const GrpTab<YsArgs<float2>>* t, int nblk, size_t smem) {
-    ys_grp_t(st, kind, t, nblk, smem);
+    launch_pdl(k_ys_pair<S>, ys_member_grid(c, sizeof(S)), dim3(64), yp_smem(c.ny, sizeof(S)), st, c.ny, c.nx / 2 + 1,
+               c.nz, m.am2ph, m.ap2ph, spec, fac);
 }
 void launch_ysolve_fac(cudaStream_t st, const DConst& c, const DMetric& m, double2* spec, const double* fac) {
     ysolve_fac_t(st, c, m, spec, fac);
 }
-void launch_ysolve_fac_slab(cudaStream_t st, const DConst& c, const DMetric& m, double2* spec, const double* fac,
-                            int dc_here) {
-    const int M1 = c.nx / 2 + 1;
-    if (ys_kind(c) == 0)
-        launch_pdl(k_ys_staged_slab, ys_member_grid(c, 0), dim3(32), ys_smem(c, 0), st, c.ny, M1, c.nz, m.am2ph, spec,
-                   fac, dc_here);
-    else
-        launch_pdl(k_ys_global_slab, ys_member_grid(c, 1), dim3(128), 0, st, c.ny, M1, c.nz, m.am2ph,
-                   reinterpret_cast<double*>(spec), fac, dc_here);
-}
 void launch_ysolve_fac(cudaStream_t st, const DConst& c, const DMetric& m, float2* spec, const double* fac) {
     ysolve_fac_t(st, c, m, spec, fac);
+}
+void launch_ys_grp(cudaStream_t st, const GrpTab<YsArgs<double2>>* t, int nblk, size_t smem) {
+    launch_pdl(k_ys_pair_grp<double2>, dim3((unsigned)nblk), dim3(64), smem, st, t);
+}
+void launch_ys_grp(cudaStream_t st, const GrpTab<YsArgs<float2>>* t, int nblk, size_t smem) {
+    launch_pdl(k_ys_pair_grp<float2>, dim3((unsigned)nblk), dim3(64), smem, st, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -747,11 +713,15 @@ void tridiag_init() {
     cudaFuncSetAttribute(k_ysolve<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     cudaFuncSetAttribute(k_ysolve<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     cudaFuncSetAttribute(k_ysolve<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-    cudaFuncSetAttribute(k_ys_staged<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(k_ys_staged<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(k_ys_staged_grp<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(k_ys_staged_grp<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(k_ys_staged_slab, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    for (auto* k : {(const void*)k_helm<double, HY_U>, (const void*)k_helm<double, HY_U / 2>,
+                    (const void*)k_helm<float, HY_U>, (const void*)k_helm<float, HY_U / 2>,
+                    (const void*)k_helm<float, HY_U, float>, (const void*)k_helm_grp<double, HY_U>,
+                    (const void*)k_helm_grp<double, HY_U / 2>, (const void*)k_helm_grp<float, HY_U>,
+                    (const void*)k_helm_grp<float, HY_U / 2>, (const void*)k_helm_grp<float, HY_U, float>})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+    for (auto* k : {(const void*)k_ys_pair<double2>, (const void*)k_ys_pair<float2>,
+                    (const void*)k_ys_pair_grp<double2>, (const void*)k_ys_pair_grp<float2>})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
     cudaFuncSetAttribute(k_helm_factors, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
 }
 
@@ -764,9 +734,9 @@ int helm_variants() { return HELM_NVAR; }
 int helm_variants(int prec) { return prec == 2 ? HELM_NVAR + 1 : HELM_NVAR; }
 
 // pivots of the Helmholtz matrices of substeps ns0..ns0+nsub-1 for the
-// current dt (coef->dt): one thread per (substep, type) runs the forward
-// elimination of InverseTridiagonal on the coefficients of clcU1Hat /
-// clcU2Hat / clcScalar (src/m_TScheme.f90:374-380,409-420,486-492)
+// current dt (coef->dt): one thread per (substep, type, wall) eliminates its
+// half of the rows, in the order of InverseTridiagonal, on the coefficients of
+// clcU1Hat / clcU2Hat / clcScalar (src/m_TScheme.f90:374-380,409-420,486-492)
 __global__ void __launch_bounds__(32) k_helm_factors(DConst cst, DMetric m, const DCoef* __restrict__ coef, int ns0,
                                                      int nsub, double a1, double a2, double a3,
                                                      double* __restrict__ facs) {
@@ -778,7 +748,7 @@ __global__ void __launch_bounds__(32) k_helm_factors(DConst cst, DMetric m, cons
     __syncthreads();
     pdl_wait();
     pdl_trigger();
-    const int q = threadIdx.x;
+    const int q = threadIdx.x >> 1, w = threadIdx.x & 1;
     if (q >= 3 * nsub) return;
     const int ns = ns0 + q / 3, t = q % 3;
     const double alp = ns == 1 ? a1 : (ns == 2 ? a2 : a3);
@@ -787,28 +757,28 @@ __global__ void __launch_bounds__(32) k_helm_factors(DConst cst, DMetric m, cons
     const double* ap = shm + (3 * t) * L;
     const double* ac = ap + L;
     const double* am = ac + L;
+    // from wall `w` (0 the lower) to the row before the junction: r, MP, MN of
+    // helm_body; the other wall's first row couples to no wall of the table
     double* F = facs + (size_t)((ns - 1) * 3 + t) * helm_stride(ny);
-    double* FA = F;
-    double* FR = F + (ny + 2);
-    double* FW = F + 2 * (ny + 2);
-    const bool vrow1 = (t == 1);  // clcU2Hat: row 1 is the identity
-    double vecm = vrow1 ? 1.0 : __dadd_rn(-__dmul_rn(beta, ac[1]), 1.0);
-    double cprev = vrow1 ? 0.0 : -__dmul_rn(beta, ap[1]);
-    FA[0] = FR[0] = FW[0] = 0.0;
-    FA[1] = 0.0;
-    FR[1] = 1.0 / vecm;
-    FW[1] = 0.0;
-    for (int jc = 2; jc <= ny; jc++) {
-        const double arr = cprev / vecm;
-        const double a = -__dmul_rn(beta, am[jc]);
-        const double b = __dadd_rn(-__dmul_rn(beta, ac[jc]), 1.0);
-        vecm = __dsub_rn(b, __dmul_rn(a, arr));
-        FA[jc] = a;
+    double* FP = F;                  // MP
+    double* FR = F + (ny + 2);       // r
+    double* FN = F + 2 * (ny + 2);   // MN
+    const int h = ny >> 1, dj = w ? -1 : 1, n = w ? ny - h : h;
+    const double* ab = w ? ap : am;  // to the row before, to the row after
+    const double* an = w ? am : ap;
+    int jc = w ? ny : 1;
+    double cprev = 0.0, vecm = 1.0;
+    for (int i = 0; i < n; i++, jc += dj) {
+        const bool one = t == 1 && jc == 1;  // clcU2Hat: row 1 is the identity
+        const double arr = i ? cprev / vecm : 0.0;
+        const double a = one ? 0.0 : -__dmul_rn(beta, ab[jc]);
+        const double b = one ? 1.0 : __dadd_rn(-__dmul_rn(beta, ac[jc]), 1.0);
+        vecm = i ? __dsub_rn(b, __dmul_rn(a, arr)) : b;
+        cprev = one ? 0.0 : -__dmul_rn(beta, an[jc]);
         FR[jc] = 1.0 / vecm;
-        FW[jc] = arr;
-        cprev = -__dmul_rn(beta, ap[jc]);
+        FP[jc] = i ? a / vecm : 0.0;
+        FN[jc] = cprev / vecm;
     }
-    FA[ny + 1] = FR[ny + 1] = FW[ny + 1] = 0.0;
 }
 
 void launch_helm_factors(cudaStream_t st, const DConst& c, const DMetric& m, const DCoef* coef, int ns0, int nsub,
@@ -817,18 +787,27 @@ void launch_helm_factors(cudaStream_t st, const DConst& c, const DMetric& m, con
                alp[0], alp[1], alp[2], fac);
 }
 
-static dim3 helm_grid(const DConst& c, int ncomp) { return dim3((c.nx + 127) / 128, c.nz, ncomp); }
-// the grouped launch's shape (32 columns x 4 z planes per CTA)
-dim3 helm_member_grid(const DConst& c, int ncomp) { return dim3((c.nx + 31) / 32, (c.nz + 3) / 4, ncomp); }
-size_t helm_smem(const DConst& c) { return helm_stride(c.ny) * sizeof(double); }
+// the launch shapes by helm_var: rows per chunk HY_U, half of that, or (FP32
+// storage) HY_U with float sweeps
+static bool helm_float(const DConst& c, int vsize) { return c.helm_var == 2 && vsize == 4; }
+size_t helm_smem(const DConst& c, int vsize) {
+    return 2 * (size_t)helm_half(c.ny - c.ny / 2, vsize, helm_float(c, vsize) ? 4 : 8);
+}
+// a CTA per work item up to the CTAs the device holds at once (8 per SM by
+// registers, fewer by shared memory), which then walk the items
+dim3 helm_member_grid(const DConst& c, int ncomp, int vsize) {
+    const long long items = ((long long)c.nx * c.nz + 31) / 32 * ncomp;
+    const int per_sm = (int)std::min<size_t>(8, (size_t)(224 * 1024) / (helm_smem(c, vsize) + 3072));
+    return dim3((unsigned)std::min<long long>(items, (long long)std::max(1, per_sm) * (c.nsm > 0 ? c.nsm : 148)));
+}
 
 template <class V>
 static void helm_grp_t(cudaStream_t st, const DConst& key, const GrpTab<HelmArgs<V>>* t, int nblk, size_t smem) {
-    constexpr int H0 = sizeof(V) == 4 ? 2 * HY_U : HY_U;
-    using WF = std::conditional_t<sizeof(V) == 4, float, double>;  // helm_var 2: float sweeps (FP32 storage)
-    if (key.helm_var == 1) launch_pdl(k_helm_grp<V, H0 / 2>, dim3((unsigned)nblk), dim3(32, 4), smem, st, t);
-    else if (key.helm_var == 2) launch_pdl(k_helm_grp<V, H0, WF>, dim3((unsigned)nblk), dim3(32, 4), smem, st, t);
-    else launch_pdl(k_helm_grp<V, H0>, dim3((unsigned)nblk), dim3(32, 4), smem, st, t);
+    using WF = std::conditional_t<sizeof(V) == 4, float, double>;
+    const dim3 g((unsigned)nblk), b(64);
+    if (key.helm_var == 1) launch_pdl(k_helm_grp<V, HY_U / 2>, g, b, smem, st, t);
+    else if (helm_float(key, sizeof(V))) launch_pdl(k_helm_grp<V, HY_U, WF>, g, b, smem, st, t);
+    else launch_pdl(k_helm_grp<V, HY_U>, g, b, smem, st, t);
 }
 void launch_helm_grp(cudaStream_t st, const DConst& key, const GrpTab<HelmArgs<double>>* t, int nblk, size_t smem) {
     helm_grp_t(st, key, t, nblk, smem);
@@ -840,37 +819,24 @@ void launch_helm_grp(cudaStream_t st, const DConst& key, const GrpTab<HelmArgs<f
 template <class V>
 static void helm_dispatch(cudaStream_t st, const DConst& c, const DCoef* coef, int comp0, int ncomp,
                           const FieldSet<V>& f, const double* duy_ym, const double* uy_ym, const double* fac) {
-    dim3 blk(32, 4);
-    dim3 grd = helm_grid(c, ncomp);
-    // rows per chunk: FP64 8 (variant 1: 4); float storage, whose ring takes
-    // half the registers, 16 (variant 1: 8)
-    constexpr int H0 = sizeof(V) == 4 ? 2 * HY_U : HY_U;
-    using WF = std::conditional_t<sizeof(V) == 4, float, double>;  // helm_var 2: float sweeps (FP32 storage)
+    using WF = std::conditional_t<sizeof(V) == 4, float, double>;
+    const dim3 g = helm_member_grid(c, ncomp, sizeof(V)), b(64);
+    const size_t smem = helm_smem(c, sizeof(V));
     if (c.helm_var == 1)
-        launch_pdl(k_helm<V, H0 / 2>, grd, blk, helm_stride(c.ny) * sizeof(double), st, c, coef, comp0, f, duy_ym,
-                   uy_ym, fac);
-    else if (c.helm_var == 2)
-        launch_pdl(k_helm<V, H0, WF>, grd, blk, helm_stride(c.ny) * sizeof(double), st, c, coef, comp0, f, duy_ym,
-                   uy_ym, fac);
+        launch_pdl(k_helm<V, HY_U / 2>, g, b, smem, st, c, coef, comp0, ncomp, f, duy_ym, uy_ym, fac);
+    else if (helm_float(c, sizeof(V)))
+        launch_pdl(k_helm<V, HY_U, WF>, g, b, smem, st, c, coef, comp0, ncomp, f, duy_ym, uy_ym, fac);
     else
-        launch_pdl(k_helm<V, H0>, grd, blk, helm_stride(c.ny) * sizeof(double), st, c, coef, comp0, f, duy_ym,
-                   uy_ym, fac);
+        launch_pdl(k_helm<V, HY_U>, g, b, smem, st, c, coef, comp0, ncomp, f, duy_ym, uy_ym, fac);
 }
 
 void launch_helm(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields& f, const double* duy_ym,
                  const double* uy_ym, const double* fac) {
-    helm_dispatch(st, c, coef, 0, 3, f, duy_ym, uy_ym, fac);
+    helm_dispatch(st, c, coef, 0, c.scalar_on ? 4 : 3, f, duy_ym, uy_ym, fac);
 }
 void launch_helm(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields32& f, const double* duy_ym,
                  const double* uy_ym, const double* fac) {
-    helm_dispatch(st, c, coef, 0, 3, f, duy_ym, uy_ym, fac);
-}
-
-void launch_helm_scalar(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields& f, const double* fac) {
-    helm_dispatch(st, c, coef, 3, 1, f, nullptr, nullptr, fac);
-}
-void launch_helm_scalar(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields32& f, const double* fac) {
-    helm_dispatch(st, c, coef, 3, 1, f, nullptr, nullptr, fac);
+    helm_dispatch(st, c, coef, 0, c.scalar_on ? 4 : 3, f, duy_ym, uy_ym, fac);
 }
 
 void launch_ysolve(cudaStream_t st, const DConst& c, const DMetric& m, double2* spec) {

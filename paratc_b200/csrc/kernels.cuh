@@ -96,22 +96,20 @@ int rhs_variants();          // compiled FP64 right-hand-side launch shapes (DCo
 int rhs_variants(int prec);  // the shapes of precision form prec (PARATC_PREC_*): FP64 3, FP32 storage 2, mixed 1
 void launch_helm_factors(cudaStream_t st, const DConst& c, const DMetric& m, const DCoef* coef, int ns0, int nsub,
                          const double* alp, double* fac);
+// u, v, w and, with scalar_on, the scalar in one launch
 void launch_helm(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields& f, const double* duy_ym,
                  const double* uy_ym, const double* fac);
 void launch_helm(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields32& f, const double* duy_ym,
                  const double* uy_ym, const double* fac);
-void launch_helm_scalar(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields& f, const double* fac);
-void launch_helm_scalar(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields32& f, const double* fac);
 void launch_ysolve(cudaStream_t st, const DConst& c, const DMetric& m, double2* spec);
 
 // k_tridiag.cu: spectral y-solve with the pivots computed once per context
-void launch_pois_factors(cudaStream_t st, const DConst& c, const DMetric& m, double* fac);
-// a z-slab rank's x-mode slab (dc_here: its column 0 is kx = kz = 0)
-void launch_pois_factors_slab(cudaStream_t st, const DConst& c, const DMetric& m, double* fac, int dc_here);
-void launch_ysolve_fac_slab(cudaStream_t st, const DConst& c, const DMetric& m, double2* spec, const double* fac,
-                            int dc_here);
+// (dc_here: column 0 is the kx = kz = 0 system; false for a z-slab rank whose
+// modes start above kx = 0)
+size_t pois_fac_doubles(const DConst& c);
+void launch_pois_factors(cudaStream_t st, const DConst& c, const DMetric& m, double* fac, int dc_here = 1);
 void launch_ysolve_fac(cudaStream_t st, const DConst& c, const DMetric& m, double2* spec, const double* fac);
-// FP32 storage form: the streaming solve on a float2 spectrum, FP64 sweeps and pivots
+// FP32 storage form: a float2 spectrum, FP64 sweeps and pivots
 void launch_ysolve_fac(cudaStream_t st, const DConst& c, const DMetric& m, float2* spec, const double* fac);
 
 // k_stats.cu: clcStat accumulation
@@ -252,12 +250,12 @@ struct RhsArgs {  // k_rhs_tile
     int pad;
 };
 template <class V>
-struct HelmArgs {  // k_helm, components comp0 .. comp0 + grid z - 1
+struct HelmArgs {  // k_helm, components comp0 .. comp0 + ncomp - 1
     DConst c;
     const DCoef* coef;
     FieldSet<V> fl;
     const double *duy_ym, *uy_ym, *fac;
-    int comp0;
+    int comp0, ncomp;
 };
 template <class V, class S>
 struct XfArgs {  // k_xf, divergence source of the substep (mode 0)
@@ -278,9 +276,9 @@ struct ZtArgs {  // k_zt
     const double2* tw;
 };
 template <class S>
-struct YsArgs {  // k_ys_staged / k_ys_global
+struct YsArgs {  // k_ys_pair
     int ny, M1, nz;
-    const double* am2ph;
+    const double *am2ph, *ap2ph;
     S* spec;
     const double* fac;
 };
@@ -320,16 +318,15 @@ long long rhs_work_rows(const DConst& c);  // (tile, row) work items of the righ
 int rhs_wave(const DConst& c);             // resident right-hand-side CTAs of the device
 void launch_rhs_grp(cudaStream_t st, const DConst& key, const GrpTab<RhsArgs<double>>* t, int nblk, int ns);
 void launch_rhs_grp(cudaStream_t st, const DConst& key, const GrpTab<RhsArgs<float>>* t, int nblk, int ns);
-dim3 helm_member_grid(const DConst& c, int ncomp);
-size_t helm_smem(const DConst& c);
+dim3 helm_member_grid(const DConst& c, int ncomp, int vsize);  // vsize: bytes of a stored value
+size_t helm_smem(const DConst& c, int vsize);
 void launch_helm_grp(cudaStream_t st, const DConst& key, const GrpTab<HelmArgs<double>>* t, int nblk, size_t smem);
 void launch_helm_grp(cudaStream_t st, const DConst& key, const GrpTab<HelmArgs<float>>* t, int nblk, size_t smem);
-// the y-solve: kind 0 staged, 1 streaming (ys_kind), per member
-int ys_kind(const DConst& c);
-dim3 ys_member_grid(const DConst& c, int kind);
-size_t ys_smem(const DConst& c, int kind);
-void launch_ys_grp(cudaStream_t st, int kind, const GrpTab<YsArgs<double2>>* t, int nblk, size_t smem);
-void launch_ys_grp(cudaStream_t st, int kind, const GrpTab<YsArgs<float2>>* t, int nblk, size_t smem);
+// the y-solve (esize: bytes of a complex value of the spectrum)
+dim3 ys_member_grid(const DConst& c, int esize);
+size_t ys_smem(const DConst& c, int esize);
+void launch_ys_grp(cudaStream_t st, const GrpTab<YsArgs<double2>>* t, int nblk, size_t smem);
+void launch_ys_grp(cudaStream_t st, const GrpTab<YsArgs<float2>>* t, int nblk, size_t smem);
 dim3 pfft_x_member_grid(const DConst& c);
 void launch_xf_grp(cudaStream_t st, int nx, const GrpTab<XfArgs<double, double2>>* t, int nblk);
 void launch_xf_grp(cudaStream_t st, int nx, const GrpTab<XfArgs<float, float2>>* t, int nblk);

@@ -42,8 +42,8 @@
 // 16-byte aligned, else the generic k_fft_x_r2c / k_fft_x_c2r; the TMA-fed z
 // transform (k_zt_tma, its tensor map encoded over the caller's x-slab)
 // where nzc has a compiled length, else the generic k_fft_z; and the
-// stored-pivot y-Thomas sweeps of the one-GPU solve (k_ys_staged /
-// k_ys_global bodies), their pivots computed once per plan for the rank's
+// stored-pivot y sweeps of the one-GPU solve (k_ys_pair), their pivots
+// computed once per plan for the rank's
 // modes (m.wnx offset to kx0; only the rank holding kx = 0 has the
 // kx = kz = 0 system with row 1 replaced by phi = 0).  The solve is the
 // same discrete system as paratc_poisson_device().
@@ -254,8 +254,6 @@ extern "C" int paratc_slab_create(const paratc_params* prm, const double* yp, in
     s->kc.nx = 2 * (s->nxl - 1);
     s->kc.ny = ny; s->kc.nz = nz; s->kc.nyp = nyp; s->kc.nyt = ny + 2;
     s->kc.nsm = s->nsm;
-    // the staged sweep copies pivot pairs as 16-byte units: an even column count
-    if ((s->nxl * nz) % 2) s->kc.solver_sel = 2;
     std::memset(&s->dm, 0, sizeof(s->dm));
     s->dm.am2ph = s->d_tab;
     s->dm.ac2ph = s->d_tab + (nyp + 1);
@@ -266,13 +264,13 @@ extern "C" int paratc_slab_create(const paratc_params* prm, const double* yp, in
     s->postx = s->twx + nx / 2;
     s->twz = s->postx + M1;
     const size_t nq = (size_t)s->nxl * nz;
-    if ((e = cudaMalloc(&s->d_fac, 2 * nq * ny * sizeof(double))) != cudaSuccess ||
+    if ((e = cudaMalloc(&s->d_fac, pois_fac_doubles(s->kc) * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc(&s->d_xslab, nq * ny * sizeof(double2))) != cudaSuccess) {
         std::fprintf(stderr, "paratc_slab_create: %s\n", cudaGetErrorString(e));
         paratc_slab_destroy(s);
         return e == cudaErrorMemoryAllocation ? PARATC_ERR_OOM : PARATC_ERR_CUDA;
     }
-    launch_pois_factors_slab(0, s->kc, s->dm, s->d_fac, s->kx0 == 0);
+    launch_pois_factors(0, s->kc, s->dm, s->d_fac, s->kx0 == 0);
     if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
         std::fprintf(stderr, "paratc_slab_create: %s\n", cudaGetErrorString(e));
         paratc_slab_destroy(s);
@@ -336,7 +334,7 @@ extern "C" int paratc_slab_middle(paratc_slab* s, double* d_xslab, void* stream)
     const bool zt = s->zt && s->zt_for == xs;
     if (zt) launch_zt_tma(st, -1, ncol, s->nz, s->zt_map, s->twz, s->nsm, s->d_err);
     else launch_fft_z(st, -1, s->kc.nx, s->ny, s->nz, xs, s->plz, s->twz);
-    launch_ysolve_fac_slab(st, s->kc, s->dm, xs, s->d_fac, s->kx0 == 0);
+    launch_ysolve_fac(st, s->kc, s->dm, xs, s->d_fac);
     if (zt) launch_zt_tma(st, +1, ncol, s->nz, s->zt_map, s->twz, s->nsm, s->d_err);
     else launch_fft_z(st, +1, s->kc.nx, s->ny, s->nz, xs, s->plz, s->twz);
     return slab_finish("paratc_slab_middle");
