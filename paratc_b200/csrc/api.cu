@@ -726,10 +726,21 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
     kc.ubulk = prm->ubulk; kc.yly = prm->yly; kc.normfft = h.normfft; kc.dt_max = prm->dt_max; kc.cflc = prm->cflc;
     kc.sc_r1b = h.sc_r1b; kc.sc_r2b = h.sc_r2b; kc.sc_r1t = h.sc_r1t; kc.sc_r2t = h.sc_r2t;
     kc.vel_limit = prm->vel_limit; kc.div_limit = prm->div_limit;
-    for (int q = 0; q < 4; q++) { kc.fdxC[q] = (float)kc.dxC[q]; kc.fdzC[q] = (float)kc.dzC[q]; kc.fIC[q] = (float)kc.IC[q]; }
-    for (int q = 0; q < 5; q++) { kc.fdxxC[q] = (float)kc.dxxC[q]; kc.fdzzC[q] = (float)kc.dzzC[q]; }
+    for (int q = 0; q < 2; q++) {
+        const double r = q ? kc.rdz : kc.rdx;
+        kc.rk16[q] = r / 384.0;
+        kc.rk256[q] = r / 6144.0;
+        kc.rk24[q] = r / 24.0;
+        kc.rvis[q] = kc.xnu * r * r / 12.0;
+        kc.rsdf[q] = kc.sdiff * r * r / 12.0;
+        kc.frk16[q] = (float)kc.rk16[q];
+        kc.frk256[q] = (float)kc.rk256[q];
+        kc.frk24[q] = (float)kc.rk24[q];
+        kc.frvis[q] = (float)kc.rvis[q];
+        kc.frsdf[q] = (float)kc.rsdf[q];
+    }
     for (int q = 0; q < 3; q++) { kc.fgrav[q] = (float)kc.grav[q]; kc.fgev[q] = (float)kc.gev[q]; kc.ffvv[q] = (float)kc.fvv[q]; }
-    kc.fucrf = (float)kc.ucrf; kc.fxnu = (float)kc.xnu; kc.fsdiff = (float)kc.sdiff;
+    kc.fucrf = (float)kc.ucrf;
 
     // ---- device memory
     const size_t nf = ctx->nf;

@@ -51,9 +51,14 @@ struct DConst {
     double ubulk, yly, normfft, dt_max, cflc;
     double sc_r1b, sc_r2b, sc_r1t, sc_r2t;   // scalar ghost: c0 = r1b*c1 + r2b, ...
     double vel_limit, div_limit;
-    // FP32 copies of the stencil constants for the FP32 right-hand side
-    float fdxC[4], fdzC[4], fdxxC[5], fdzzC[5], fIC[4], fgrav[3], fgev[3], ffvv[3];
-    float fucrf, fxnu, fsdiff;
+    // scales of the right-hand side's whole-number stencil weights (k_rhs.cu),
+    // x then z: difference times one 16-fold interpolation (rdx / (24 16)) and
+    // two (rdx / (24 256)), plain difference (rdx / 24), viscous and scalar
+    // second difference (xnu rdx^2 / 12, sdiff rdx^2 / 12)
+    double rk16[2], rk256[2], rk24[2], rvis[2], rsdf[2];
+    // FP32 copies for the FP32 right-hand side
+    float frk16[2], frk256[2], frk24[2], frvis[2], frsdf[2], fgrav[3], fgev[3], ffvv[3];
+    float fucrf;
 };
 
 // per-substep coefficients (PMcoeUpdate, src/m_Parameters.f90:215-230) and

@@ -29,11 +29,25 @@
 // differences sum to zero over a periodic line, so they carry nothing into
 // s3tot but rounding).
 //
+// What bounds it: at 8 warps per SM (230 registers) the latency of its FP64
+// chains, its FP64 pipe half busy; a form with 12 warps (168 registers) spills
+// and took 83 us instead of 55 at 128 x 96 x 128.  So operations are saved:
+// the stencils' whole-number weights (interp16, der24, lap12) take 3, 3 and 4
+// operations instead of 4, 4 and 5 and no constants from memory; one barrier
+// per row; the histories of a row are read at its start, after an L2 prefetch
+// one row ahead, where registers for a row of them made the scalar form spill.
+// One B200, per launch, before and after: 58.4 -> 55.5 us at 128 x 96 x 128,
+// 561 -> 546 us at 384 x 192 x 256; with the scalar 51.5 -> 46.0 us at 96^3
+// and 2.79 -> 2.44 ms at 1536 x 160 x 256 (1.33 ms of memory at the copy
+// rate); FP32 storage 1.86 -> 1.80 ms there.
+//
 // The same kernel performs PMcoeUpdate (src/m_Parameters.f90:215-230),
 // Update_uy_ym (src/m_FlowCase.f90:112-122) and the flow-rate constraint
 // (src/m_TScheme.f90:269-300): every CTA writes its partial of s3tot and the
 // last CTA to finish reduces them in a fixed order and stores the uniform
 // RhsX correction and the substep coefficients for the kernels that follow.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "reduce.cuh"
@@ -44,7 +58,7 @@ namespace {
 constexpr int TX = 32, TZ = 8, HX = 4, HZ = 3;
 constexpr int SX = TX + 2 * HX;  // 40: x offsets -4 .. 35 of the tile (the stencils read -3 .. 34)
 constexpr int SZ = TZ + 2 * HZ;  // 14
-constexpr int SLAB = SX * SZ;    // 560 doubles per field and row
+constexpr int SLAB = SX * SZ;    // 560 values per field and row
 // The launch shape, per precision and compiled variant VAR (the tuner's
 // choice, paratc_autotune_all): PF rows loaded ahead beyond row j+1 (copy
 // groups in flight; FP64), ZC z-adjacent cells per thread (2 lets the shared
@@ -78,6 +92,8 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+__device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
 // the field a copy reads (f = 0 ux, 1 uy, 2 uz, 3 p, 4 scalar)
 __device__ __forceinline__ const double* field_of(const Fields& fl, int f) {
     return f == 0 ? fl.ux : f == 1 ? fl.uy : f == 2 ? fl.uz : f == 3 ? fl.pr : fl.sc;
@@ -95,6 +111,31 @@ __device__ __forceinline__ double ld_field(const FieldSet<V>& fl, int f, size_t 
     const V* q = f == 0 ? fl.ux : f == 1 ? fl.uy : f == 2 ? fl.uz : fl.sc;
     return (double)__ldg(q + off);
 }
+
+// The 4th-order stencils of src/m_MeshAndMetries.f90:96-101 with their common
+// denominators taken out, (-1 9 9 -1)/16, (1 -27 27 -1)/24 and (-1 16 -30 16
+// -1)/12: whole-number weights are immediates of the FMA, the symmetric taps
+// add first (three operations instead of four, four instead of five), and the
+// scale is one factor of the whole term.
+template <class T>
+__device__ __forceinline__ T interp16(T a, T b, T c, T d) { return fma(T(9), b + c, -(a + d)); }
+template <class T>
+__device__ __forceinline__ T der24(T a, T b, T c, T d) { return fma(T(27), c - b, a - d); }
+// Sums of products, written out as fma everywhere in this kernel, so that no
+// instantiation may fuse them another way: an ensemble's grouped launch
+// computes what a member's own launch does.
+template <class T>
+__device__ __forceinline__ T dif2(T a, T b, T c, T d) { return fma(a, b, -(c * d)); }  // a b - c d
+template <class T>
+__device__ __forceinline__ T mad2(T a, T b, T c, T d) { return fma(a, b, c * d); }  // a b + c d
+template <class T>
+__device__ __forceinline__ T mad3(T a, T b, T c, T d, T e, T f) { return fma(a, b, fma(c, d, e * f)); }
+template <class T>
+__device__ __forceinline__ T der24p(const T (&a)[4], const T (&b)[4]) {
+    return fma(T(27), dif2(a[2], b[2], a[1], b[1]), dif2(a[0], b[0], a[3], b[3]));
+}
+template <class T>
+__device__ __forceinline__ T lap12(T a, T b, T c, T d, T e) { return fma(T(16), b + d, fma(T(-30), c, -(a + e))); }
 
 __device__ __forceinline__ int modp(int i, int n) {
     int r = i % n;
@@ -136,7 +177,8 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
     __shared__ __align__(128) double smet[NB][ROWMET];
     const int lane = threadIdx.x, wq = threadIdx.y, tid = wq * 32 + lane;
     const int nx = c.nx, nz = c.nz, ny = c.ny;
-    const size_t pl = (size_t)c.nyt * nx;
+    // 32-bit element offsets: a field of 2^32 values does not fit the device
+    const unsigned pl = (unsigned)c.nyt * nx;
     // work = the (tile, row) pairs in tile-major order; block b takes the
     // contiguous range [b*W/B, (b+1)*W/B), so one wave of resident blocks
     // covers the grid with at most one row of imbalance
@@ -162,17 +204,23 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
     const double tb = 2.0 * pmBeta, tbs = 2.0 * pmBetaSc;
     // stencil constants straight from the parameter bank, in the kernel's precision
 #define KC(a64, a32, q) (F64 ? (T)c.a64[q] : (T)c.a32[q])
-#define dxC(q) KC(dxC, fdxC, q)
-#define dzC(q) KC(dzC, fdzC, q)
-#define dxxC(q) KC(dxxC, fdxxC, q)
-#define dzzC(q) KC(dzzC, fdzzC, q)
 #define grav(q) KC(grav, fgrav, q)
 #define gev(q) KC(gev, fgev, q)
+#define gev16(q) (gev(q) * T(0.0625))
+#define kx16 KC(rk16, frk16, 0)
+#define kz16 KC(rk16, frk16, 1)
+#define kx256 KC(rk256, frk256, 0)
+#define kz256 KC(rk256, frk256, 1)
+#define gx24 KC(rk24, frk24, 0)
+#define gz24 KC(rk24, frk24, 1)
+#define vx KC(rvis, frvis, 0)
+#define vz KC(rvis, frvis, 1)
+#define svx KC(rsdf, frsdf, 0)
+#define svz KC(rsdf, frsdf, 1)
 #define fvv(q) KC(fvv, ffvv, q)
-    const T I1 = KC(IC, fIC, 0), I2 = KC(IC, fIC, 1), I3 = KC(IC, fIC, 2), I4 = KC(IC, fIC, 3);
-    const T ucrf = F64 ? (T)c.ucrf : (T)c.fucrf, xnu = F64 ? (T)c.xnu : (T)c.fxnu;
+    // the scales that the whole-number stencil weights leave out
+    const T ucrf = F64 ? (T)c.ucrf : (T)c.fucrf, ucrf16 = T(16) * ucrf;
     const T tpG = (T)pmGamma, tpT = (T)pmTheta, tpA = (T)pmAlpha, ttb = (T)tb, ttbs = (T)tbs;
-    const T tsdiff = F64 ? (T)c.sdiff : (T)c.fsdiff;
     double s3 = 0.0;
 
     for (long long g = gbeg; g < gend;) {
@@ -208,7 +256,7 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
             }
         }
         // FP64: the 16-byte pairs this thread copies (the same for every field)
-        size_t gp[F64 ? NP2 : 1];
+        unsigned gp[F64 ? NP2 : 1];
         int sp[F64 ? NP2 : 1];
         bool vp[F64 ? NP2 : 1];
         if constexpr (F64) {
@@ -217,17 +265,17 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
                 const int e = tid + q * NTHR;
                 vp[q] = e < NPR;
                 const int zz = e / NPAIR, pp = e - zz * NPAIR;
-                gp[q] = (size_t)modp(k0 - HZ + zz, nz) * pl + (size_t)modp(i0 - HX + 2 * pp, nx);
+                gp[q] = (unsigned)modp(k0 - HZ + zz, nz) * pl + (unsigned)modp(i0 - HX + 2 * pp, nx);
                 sp[q] = zz * SX + 2 * pp;
             }
         }
 #define LOAD_ROW64(jrow)                                                                             \
     do {                                                                                             \
         double* dst_ = reinterpret_cast<double*>(sm) + (size_t)((jrow) % NB) * NF * SLAB;           \
-        const size_t ro_ = (size_t)(jrow) * nx;                                                      \
+        const unsigned ro_ = (unsigned)(jrow) * nx;                                                  \
         _Pragma("unroll") for (int f_ = 0; f_ < NF; f_++)                                            \
             _Pragma("unroll") for (int q_ = 0; q_ < NP2; q_++) if (vp[q_])                           \
-                cp_async16(dst_ + f_ * SLAB + sp[q_], field_of(fl, f_) + gp[q_] + ro_);              \
+                cp_async16(dst_ + f_ * SLAB + sp[q_], field_of(fl, f_) + (gp[q_] + ro_));            \
         if (tid < ROWMET / 2) cp_async16(&smet[(jrow) % NB][2 * tid], m.rowmet + (size_t)(jrow) * ROWMET + 2 * tid); \
     } while (0)
         // FP32: load, convert, store (FP32 storage: the float fields by
@@ -273,8 +321,9 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
         const int i = i0 + lane;
         int kk[ZC];
         bool act[ZC];
-        // explicit histories of the next row are loaded one row ahead, held
-        // in their storage type (widened where used, so the loads stay in flight)
+        // FP32 forms: explicit histories of the next row are loaded one row
+        // ahead, held in their storage type (widened where used, so the loads
+        // stay in flight)
         V hxn[ZC], hyn[ZC], hzn[ZC], hcn[ZC];
         V u64m[ZC], u64c[ZC], u64p[ZC];  // FP32 forms: ux of the own column, rows j-1, j, j+1
 #pragma unroll
@@ -291,9 +340,9 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
             u64m[cz] = u64c[cz] = u64p[cz] = 0.0;
             if (act[cz]) {
                 const size_t q = (size_t)kk[cz] * pl + (size_t)j0 * nx + i;
-                hxn[cz] = fl.hx[q]; hyn[cz] = fl.hy[q]; hzn[cz] = fl.hz[q];
-                if (SCALAR) hcn[cz] = fl.hc[q];
                 if constexpr (!F64) {
+                    hxn[cz] = fl.hx[q]; hyn[cz] = fl.hy[q]; hzn[cz] = fl.hz[q];
+                    if (SCALAR) hcn[cz] = fl.hc[q];
                     u64m[cz] = __ldg(&fl.ux[q - nx]);
                     u64c[cz] = __ldg(&fl.ux[q]);
                     u64p[cz] = __ldg(&fl.ux[q + nx]);
@@ -307,38 +356,36 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
             double pre[F64 ? 1 : NF][F64 ? 1 : NSLOT];
             double mpre = 0.0;
             const bool more = j + 2 <= j1 + 1;
-            if constexpr (F64) {
-                // the slot of row j+1+PF was last read by row j-1's arithmetic,
-                // which every thread finished at the barrier closing it
-                if (j + 1 + PF <= j1 + 1) LOAD_ROW64(j + 1 + PF);
-                cp_async_commit();
-            } else {
+            if constexpr (!F64) {
                 if (more) {
                     const size_t ro = (size_t)(j + 2) * nx;
-                    T* dst = sm + (size_t)((j + 2) % NB) * NF * SLAB;
 #pragma unroll
                     for (int f = 0; f < NF; f++) {
-                        if (F32S && f != 3) {
-                            // the slot of row j+2 was last read by row j-2's arithmetic
-#pragma unroll
-                            for (int s4 = 0; s4 < NQ2; s4++)
-                                if (vq[s4]) cp_async16(dst + f * SLAB + sq[s4], fieldv(fl, f) + gq[s4] + ro);
-                            continue;
-                        }
+                        if (F32S && f != 3) continue;  // copied by cp.async below
 #pragma unroll
                         for (int sl = 0; sl < NSLOT; sl++)
                             pre[f][sl] = sval[sl] ? ld_field(fl, f, goff[sl] + ro) : 0.0;
                     }
                     if (tid < ROWMET) mpre = __ldg(m.rowmet + (size_t)(j + 2) * ROWMET + tid);
                 }
-                if constexpr (F32S) cp_async_commit();  // one group per row, empty or not
             }
             V hx0a[ZC], hy0a[ZC], hz0a[ZC], hc0a[ZC];
-            size_t q0a[ZC];
+            unsigned q0a[ZC];
 #pragma unroll
             for (int cz = 0; cz < ZC; cz++) {
+                q0a[cz] = (unsigned)kk[cz] * pl + (unsigned)j * nx + i;
+                if constexpr (F64) {  // in flight until the end of the row's arithmetic
+                    if (act[cz]) {
+                        hx0a[cz] = fl.hx[q0a[cz]]; hy0a[cz] = fl.hy[q0a[cz]]; hz0a[cz] = fl.hz[q0a[cz]];
+                        if (SCALAR) hc0a[cz] = fl.hc[q0a[cz]];
+                        // the next row's into L2 (a register per value would spill)
+                        const unsigned qn = q0a[cz] + nx;
+                        l2_prefetch(fl.hx + qn); l2_prefetch(fl.hy + qn); l2_prefetch(fl.hz + qn);
+                        if (SCALAR) l2_prefetch(fl.hc + qn);
+                    }
+                    continue;
+                }
                 hx0a[cz] = hxn[cz]; hy0a[cz] = hyn[cz]; hz0a[cz] = hzn[cz]; hc0a[cz] = hcn[cz];
-                q0a[cz] = (size_t)kk[cz] * pl + (size_t)j * nx + i;
                 if (act[cz] && j + 1 <= j1) {
                     hxn[cz] = fl.hx[q0a[cz] + nx]; hyn[cz] = fl.hy[q0a[cz] + nx]; hzn[cz] = fl.hz[q0a[cz] + nx];
                     if (SCALAR) hcn[cz] = fl.hc[q0a[cz] + nx];
@@ -349,12 +396,28 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
 #pragma unroll
             for (int cz = 0; cz < ZC; cz++)
                 u64n[cz] = (!F64 && act[cz] && j + 2 <= ny + 1) ? __ldg(&fl.ux[q0a[cz] + 2 * nx]) : (V)0;
+            // the row's one barrier: row j+1 is there for every thread, and every
+            // thread has finished row j-1's arithmetic, the last to read the slot
+            // that the next copies go to (row j-2's)
+            if constexpr (F64) cp_async_wait<PF - 1>();
+            else if constexpr (F32S) cp_async_wait<0>();
+            __syncthreads();
             if constexpr (F64) {
-                cp_async_wait<PF>();  // the group holding row j+1 is complete
-                __syncthreads();
+                if (j + 1 + PF <= j1 + 1) LOAD_ROW64(j + 1 + PF);
+                cp_async_commit();  // one group per row, empty or not
             } else if constexpr (F32S) {
-                cp_async_wait<1>();  // row j+1's quads (the newest group is row j+2's)
-                __syncthreads();
+                if (more) {
+                    const size_t ro = (size_t)(j + 2) * nx;
+                    T* dst = sm + (size_t)((j + 2) % NB) * NF * SLAB;
+#pragma unroll
+                    for (int f = 0; f < NF; f++) {
+                        if (f == 3) continue;
+#pragma unroll
+                        for (int s4 = 0; s4 < NQ2; s4++)
+                            if (vq[s4]) cp_async16(dst + f * SLAB + sq[s4], fieldv(fl, f) + gq[s4] + ro);
+                    }
+                }
+                cp_async_commit();
             }
             // both cells are computed before any global store, so that the
             // compiler may load a tap the two cells share once
@@ -364,141 +427,138 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
                 const T* Sc = sm + (size_t)(j % NB) * NF * SLAB;
                 const T* Sp = sm + (size_t)((j + 1) % NB) * NF * SLAB;
 #define V(S, f, dx, dz) (S)[(f) * SLAB + (w + HZ + (dz)) * SX + (lane + HX + (dx))]
+// 16 x the 4-point interpolation of field f along x at offset dx (o = 0: of
+// the points dx-2 .. dx+1, 1: of dx-1 .. dx+2) and z plane dz, and along z at
+// offset dz; 12 dx^2 (dz^2) x the second difference; 24 dx x the difference
+// of four values
+#define XI(S, f, dx, o, dz) \
+    interp16(V(S, f, (dx) - 2 + (o), dz), V(S, f, (dx) - 1 + (o), dz), V(S, f, (dx) + (o), dz), V(S, f, (dx) + 1 + (o), dz))
+#define ZI(S, f, dx, dz) interp16(V(S, f, dx, (dz) - 2), V(S, f, dx, (dz) - 1), V(S, f, dx, dz), V(S, f, dx, (dz) + 1))
+#define XL(S, f) lap12(V(S, f, -2, 0), V(S, f, -1, 0), V(S, f, 0, 0), V(S, f, 1, 0), V(S, f, 2, 0))
+#define ZL(S, f) lap12(V(S, f, 0, -2), V(S, f, 0, -1), V(S, f, 0, 0), V(S, f, 0, 1), V(S, f, 0, 2))
             const bool top = (j == ny);
             const double* M = smet[j % NB];
 #define MET(q) M[q]
             const double IY1d = MET(0), IY3d = MET(1);
             const T IY1 = (T)IY1d, IY2 = (T)(1.0 - IY1d), IY3 = (T)IY3d, IY4 = (T)(1.0 - IY3d);
-            const T rdyp = (T)MET(2), rdyc = (T)MET(3);
+            const T rdyp = (T)MET(2), rdyc = (T)MET(3), rdyp16 = T(0.0625) * rdyp;
             const double dyp = MET(4);
             const T ap2c = (T)MET(5), ac2c = (T)MET(6), am2c = (T)MET(7);
 #pragma unroll
             for (int cz = 0; cz < ZC; cz++) {
             const int w = wq * ZC + cz;
-            const T hx0 = (T)hx0a[cz], hy0 = (T)hy0a[cz], hz0 = (T)hz0a[cz], hc0 = (T)hc0a[cz];
-            (void)hc0;
 
             // ---------------- RhsX (:169-204)
             T conv_x, rhs_x;
             {
                 const T uxc = V(Sc, 0, 0, 0), uxjm = V(Sm, 0, 0, 0), uxjp = V(Sp, 0, 0, 0);
-                const T uxhyc = IY1 * uxjm + IY2 * uxc;
-                const T uxhyp = IY3 * uxc + IY4 * uxjp;
-                T h11 = 0;
+                const T uxhyc = mad2(IY1, uxjm, IY2, uxc);
+                const T uxhyp = mad2(IY3, uxc, IY4, uxjp);
+                T u1[4], z3[4], x3[4];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {  // uxhx at x offsets -2..1
-                    const int d = q - 2;
-                    const T uh = I1 * V(Sc, 0, d - 1, 0) + I2 * V(Sc, 0, d, 0) + I3 * V(Sc, 0, d + 1, 0) + I4 * V(Sc, 0, d + 2, 0);
-                    h11 = (q == 0) ? dxC(0) * uh * (uh + ucrf) : h11 + dxC(q) * uh * (uh + ucrf);
+                for (int q = 0; q < 4; q++) {
+                    u1[q] = XI(Sc, 0, q - 2, 1, 0);  // uxhx at x offsets -2..1
+                    z3[q] = ZI(Sc, 0, 0, q - 1);     // uxhz, uzhx at z offsets -1..2
+                    x3[q] = XI(Sc, 2, 0, 0, q - 1);
                 }
-                const T uyhx_j = I1 * V(Sc, 1, -2, 0) + I2 * V(Sc, 1, -1, 0) + I3 * V(Sc, 1, 0, 0) + I4 * V(Sc, 1, 1, 0);
-                const T uyhx_p = top ? T(0) : I1 * V(Sp, 1, -2, 0) + I2 * V(Sp, 1, -1, 0) + I3 * V(Sp, 1, 0, 0) + I4 * V(Sp, 1, 1, 0);
-                const T h12 = (uyhx_p * uxhyp - uyhx_j * uxhyc) * rdyp;
-                T h13 = 0;
-#pragma unroll
-                for (int q = 0; q < 4; q++) {  // z offsets -1..2
-                    const int d = q - 1;
-                    const T uxhz = I1 * V(Sc, 0, 0, d - 2) + I2 * V(Sc, 0, 0, d - 1) + I3 * V(Sc, 0, 0, d) + I4 * V(Sc, 0, 0, d + 1);
-                    const T uzhx = I1 * V(Sc, 2, -2, d) + I2 * V(Sc, 2, -1, d) + I3 * V(Sc, 2, 0, d) + I4 * V(Sc, 2, 1, d);
-                    h13 = (q == 0) ? dzC(0) * uxhz * uzhx : h13 + dzC(q) * uxhz * uzhx;
-                }
-                const T d11 = dxxC(0) * V(Sc, 0, -2, 0) + dxxC(1) * V(Sc, 0, -1, 0) + dxxC(2) * uxc + dxxC(3) * V(Sc, 0, 1, 0) + dxxC(4) * V(Sc, 0, 2, 0);
-                const T d22 = ap2c * uxjp + ac2c * uxc + am2c * uxjm;
-                const T d33 = dzzC(0) * V(Sc, 0, 0, -2) + dzzC(1) * V(Sc, 0, 0, -1) + dzzC(2) * uxc + dzzC(3) * V(Sc, 0, 0, 1) + dzzC(4) * V(Sc, 0, 0, 2);
-                const T dcq13 = d11 + d33;
+                const T f1[4] = {u1[0] + ucrf16, u1[1] + ucrf16, u1[2] + ucrf16, u1[3] + ucrf16};
+                const T uyhx_j = XI(Sc, 1, 0, 0, 0);
+                const T uyhx_p = top ? T(0) : XI(Sp, 1, 0, 0, 0);
+                const T d22 = mad3(ap2c, uxjp, ac2c, uxc, am2c, uxjm);
                 if constexpr (F64) {
-                    if (act[cz]) s3 += SCALAR ? uxc * dyp : (dcq13 + d22) * dyp;
+                    if (act[cz]) s3 = fma(SCALAR ? uxc : d22, dyp, s3);
                 } else if (act[cz]) {
                     s3 += SCALAR ? u64c[cz] * dyp
                                  : (MET(5) * u64p[cz] + MET(6) * u64c[cz] + MET(7) * u64m[cz]) * dyp;
                 }
-                conv_x = -h11 - h12 - h13 + xnu * dcq13 + grav(0);
-                const T gradp = dxC(0) * V(Sc, 3, -2, 0) + dxC(1) * V(Sc, 3, -1, 0) + dxC(2) * V(Sc, 3, 0, 0) + dxC(3) * V(Sc, 3, 1, 0);
-                rhs_x = tpG * conv_x + tpT * hx0 - tpA * gradp + ttb * d22;
+                T cv = fma(-dif2(uyhx_p, uxhyp, uyhx_j, uxhyc), rdyp16, grav(0));
+                cv = fma(-kz256, der24p(z3, x3), cv);
+                cv = fma(-kx256, der24p(u1, f1), cv);
+                conv_x = fma(vx, XL(Sc, 0), fma(vz, ZL(Sc, 0), cv));
+                const T gp = der24(V(Sc, 3, -2, 0), V(Sc, 3, -1, 0), V(Sc, 3, 0, 0), V(Sc, 3, 1, 0));
+                rhs_x = fma(tpG, conv_x, fma(-(tpA * gx24), gp, ttb * d22));
             }
             // ---------------- RhsY (:206-236)
             T conv_y, rhs_y;
             {
-                const T qsucac = T(0.25) * rdyc;
-                T h21 = 0.0, h23 = 0.0;
+                T x1[4], u1[4], z3[4], w3[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {  // offsets -1..2
                     const int d = q - 1;
-                    const T uxh = IY1 * V(Sm, 0, d, 0) + IY2 * V(Sc, 0, d, 0) + ucrf;
-                    const T uzh = IY1 * V(Sm, 2, 0, d) + IY2 * V(Sc, 2, 0, d);
-                    const T uyhx = I1 * V(Sc, 1, d - 2, 0) + I2 * V(Sc, 1, d - 1, 0) + I3 * V(Sc, 1, d, 0) + I4 * V(Sc, 1, d + 1, 0);
-                    const T uyhz = I1 * V(Sc, 1, 0, d - 2) + I2 * V(Sc, 1, 0, d - 1) + I3 * V(Sc, 1, 0, d) + I4 * V(Sc, 1, 0, d + 1);
-                    h21 = (q == 0) ? dxC(0) * uyhx * uxh : h21 + dxC(q) * uyhx * uxh;
-                    h23 = (q == 0) ? dzC(0) * uyhz * uzh : h23 + dzC(q) * uyhz * uzh;
+                    x1[q] = XI(Sc, 1, d, 0, 0);
+                    u1[q] = fma(IY1, V(Sm, 0, d, 0), fma(IY2, V(Sc, 0, d, 0), ucrf));
+                    z3[q] = ZI(Sc, 1, 0, d);
+                    w3[q] = mad2(IY1, V(Sm, 2, 0, d), IY2, V(Sc, 2, 0, d));
                 }
                 const T vp = V(Sp, 1, 0, 0), vc = V(Sc, 1, 0, 0), vm = V(Sm, 1, 0, 0);
-                const T h22 = ((vp + vc) * (vp + vc) - (vc + vm) * (vc + vm)) * qsucac;
-                const T d11 = dxxC(0) * V(Sc, 1, -2, 0) + dxxC(1) * V(Sc, 1, -1, 0) + dxxC(2) * vc + dxxC(3) * V(Sc, 1, 1, 0) + dxxC(4) * V(Sc, 1, 2, 0);
-                const T d22 = (T)MET(8) * vp + (T)MET(9) * vc + (T)MET(10) * vm;
-                const T d33 = dzzC(0) * V(Sc, 1, 0, -2) + dzzC(1) * V(Sc, 1, 0, -1) + dzzC(2) * vc + dzzC(3) * V(Sc, 1, 0, 1) + dzzC(4) * V(Sc, 1, 0, 2);
-                conv_y = -h21 - h22 - h23 + xnu * (d11 + d33) + grav(1);
-                const T gradp = (V(Sc, 3, 0, 0) - V(Sm, 3, 0, 0)) * rdyc;
-                rhs_y = tpG * conv_y + tpT * hy0 - tpA * gradp + ttb * d22;
+                // (vp + vc)^2 - (vc + vm)^2 = (vp - vm) (vp + 2 vc + vm)
+                const T h22 = (vp - vm) * fma(T(2), vc, vp + vm);
+                const T d22 = mad3((T)MET(8), vp, (T)MET(9), vc, (T)MET(10), vm);
+                T cv = fma(-h22, T(0.25) * rdyc, grav(1));
+                cv = fma(-kz16, der24p(z3, w3), cv);
+                cv = fma(-kx16, der24p(x1, u1), cv);
+                conv_y = fma(vx, XL(Sc, 1), fma(vz, ZL(Sc, 1), cv));
+                const T gradp = V(Sc, 3, 0, 0) - V(Sm, 3, 0, 0);
+                rhs_y = fma(tpG, conv_y, fma(-(tpA * rdyc), gradp, ttb * d22));
             }
             // ---------------- RhsZ (:238-267)
             T conv_z, rhs_z;
             {
                 const T uzc = V(Sc, 2, 0, 0);
-                const T uzhyc = IY1 * V(Sm, 2, 0, 0) + IY2 * uzc;
-                const T uzhyp = IY3 * uzc + IY4 * V(Sp, 2, 0, 0);
-                T h31 = 0.0, h33 = 0.0;
+                const T uzhyc = mad2(IY1, V(Sm, 2, 0, 0), IY2, uzc);
+                const T uzhyp = mad2(IY3, uzc, IY4, V(Sp, 2, 0, 0));
+                T x1[4], z1[4], w3[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const int d = q - 1;  // x offsets -1..2 for h31
-                    const T uzhx = I1 * V(Sc, 2, d - 2, 0) + I2 * V(Sc, 2, d - 1, 0) + I3 * V(Sc, 2, d, 0) + I4 * V(Sc, 2, d + 1, 0);
-                    const T uxhz = I1 * V(Sc, 0, d, -2) + I2 * V(Sc, 0, d, -1) + I3 * V(Sc, 0, d, 0) + I4 * V(Sc, 0, d, 1);
-                    h31 = (q == 0) ? dxC(0) * uzhx * (uxhz + ucrf) : h31 + dxC(q) * uzhx * (uxhz + ucrf);
-                    const int e = q - 2;  // z offsets -2..1 for h33
-                    const T uzhz = I1 * V(Sc, 2, 0, e - 1) + I2 * V(Sc, 2, 0, e) + I3 * V(Sc, 2, 0, e + 1) + I4 * V(Sc, 2, 0, e + 2);
-                    h33 = (q == 0) ? dzC(0) * uzhz * uzhz : h33 + dzC(q) * uzhz * uzhz;
+                    const int d = q - 1;  // x offsets -1..2
+                    x1[q] = XI(Sc, 2, d, 0, 0);
+                    z1[q] = ZI(Sc, 0, d, 0) + ucrf16;
+                    w3[q] = ZI(Sc, 2, 0, d);  // uzhz at z offsets -2..1
                 }
-                const T uyhz_j = I1 * V(Sc, 1, 0, -2) + I2 * V(Sc, 1, 0, -1) + I3 * V(Sc, 1, 0, 0) + I4 * V(Sc, 1, 0, 1);
-                const T uyhz_p = top ? T(0) : I1 * V(Sp, 1, 0, -2) + I2 * V(Sp, 1, 0, -1) + I3 * V(Sp, 1, 0, 0) + I4 * V(Sp, 1, 0, 1);
-                const T h32 = (uyhz_p * uzhyp - uyhz_j * uzhyc) * rdyp;
-                const T d11 = dxxC(0) * V(Sc, 2, -2, 0) + dxxC(1) * V(Sc, 2, -1, 0) + dxxC(2) * uzc + dxxC(3) * V(Sc, 2, 1, 0) + dxxC(4) * V(Sc, 2, 2, 0);
-                const T d22 = ap2c * V(Sp, 2, 0, 0) + ac2c * uzc + am2c * V(Sm, 2, 0, 0);
-                const T d33 = dzzC(0) * V(Sc, 2, 0, -2) + dzzC(1) * V(Sc, 2, 0, -1) + dzzC(2) * uzc + dzzC(3) * V(Sc, 2, 0, 1) + dzzC(4) * V(Sc, 2, 0, 2);
-                conv_z = -h31 - h32 - h33 + xnu * (d11 + d33) + grav(2);
-                const T gradp = dzC(0) * V(Sc, 3, 0, -2) + dzC(1) * V(Sc, 3, 0, -1) + dzC(2) * V(Sc, 3, 0, 0) + dzC(3) * V(Sc, 3, 0, 1);
-                rhs_z = tpG * conv_z + tpT * hz0 - tpA * gradp + ttb * d22;
+                const T uyhz_j = ZI(Sc, 1, 0, 0);
+                const T uyhz_p = top ? T(0) : ZI(Sp, 1, 0, 0);
+                const T d22 = mad3(ap2c, V(Sp, 2, 0, 0), ac2c, uzc, am2c, V(Sm, 2, 0, 0));
+                T cv = fma(-dif2(uyhz_p, uzhyp, uyhz_j, uzhyc), rdyp16, grav(2));
+                cv = fma(-kz256, der24p(w3, w3), cv);
+                cv = fma(-kx256, der24p(x1, z1), cv);
+                conv_z = fma(vx, XL(Sc, 2), fma(vz, ZL(Sc, 2), cv));
+                const T gp = der24(V(Sc, 3, 0, -2), V(Sc, 3, 0, -1), V(Sc, 3, 0, 0), V(Sc, 3, 0, 1));
+                rhs_z = fma(tpG, conv_z, fma(-(tpA * gz24), gp, ttb * d22));
             }
             if (SCALAR) {
                 // ---------------- scalar transport (:302-357)
                 const T scc = V(Sc, 4, 0, 0), scjm = V(Sm, 4, 0, 0), scjp = V(Sp, 4, 0, 0);
-                const T shyc = IY1 * scjm + IY2 * scc;
-                const T shyp = IY3 * scc + IY4 * scjp;
-                T hc1 = 0, hc3 = 0, shx0 = 0, shz0 = 0;
+                const T shyc = mad2(IY1, scjm, IY2, scc);
+                const T shyp = mad2(IY3, scc, IY4, scjp);
+                T u1[4], x1[4], w3[4], z3[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const int d = q - 1;
-                    const T shx = I1 * V(Sc, 4, d - 2, 0) + I2 * V(Sc, 4, d - 1, 0) + I3 * V(Sc, 4, d, 0) + I4 * V(Sc, 4, d + 1, 0);
-                    const T shz = I1 * V(Sc, 4, 0, d - 2) + I2 * V(Sc, 4, 0, d - 1) + I3 * V(Sc, 4, 0, d) + I4 * V(Sc, 4, 0, d + 1);
-                    if (q == 1) { shx0 = shx; shz0 = shz; }
-                    const T ua = V(Sc, 0, d, 0) + fvv(0);
-                    const T wa = V(Sc, 2, 0, d) + fvv(2);
-                    hc1 = (q == 0) ? dxC(0) * ua * shx : hc1 + dxC(q) * ua * shx;
-                    hc3 = (q == 0) ? dzC(0) * wa * shz : hc3 + dzC(q) * wa * shz;
+                    u1[q] = V(Sc, 0, d, 0) + fvv(0);
+                    x1[q] = XI(Sc, 4, d, 0, 0);
+                    w3[q] = V(Sc, 2, 0, d) + fvv(2);
+                    z3[q] = ZI(Sc, 4, 0, d);
                 }
-                const T c1 = gev(0) * shx0, c2 = gev(1) * shyc, c3 = gev(2) * shz0;
-                rhs_x = rhs_x + tpG * c1;
-                rhs_y = rhs_y + tpG * c2;
-                rhs_z = rhs_z + tpG * c3;
-                conv_x = conv_x + c1;
-                conv_y = conv_y + c2;
-                conv_z = conv_z + c3;
-                const T hc2 = ((V(Sp, 1, 0, 0) + fvv(1)) * shyp - (V(Sc, 1, 0, 0) + fvv(1)) * shyc) * rdyp;
-                const T d11 = dxxC(0) * V(Sc, 4, -2, 0) + dxxC(1) * V(Sc, 4, -1, 0) + dxxC(2) * scc + dxxC(3) * V(Sc, 4, 1, 0) + dxxC(4) * V(Sc, 4, 2, 0);
-                const T d22 = (T)MET(11) * scjp + (T)MET(12) * scc + (T)MET(13) * scjm;
-                const T d33 = dzzC(0) * V(Sc, 4, 0, -2) + dzzC(1) * V(Sc, 4, 0, -1) + dzzC(2) * scc + dzzC(3) * V(Sc, 4, 0, 1) + dzzC(4) * V(Sc, 4, 0, 2);
-                const T convc = -hc1 - hc2 - hc3 + tsdiff * (d11 + d33);
-                o_rc[cz] = tpG * convc + tpT * hc0 + ttbs * d22;
+                const T c1 = gev16(0) * x1[1], c2 = gev(1) * shyc, c3 = gev16(2) * z3[1];
+                rhs_x = fma(tpG, c1, rhs_x);
+                rhs_y = fma(tpG, c2, rhs_y);
+                rhs_z = fma(tpG, c3, rhs_z);
+                conv_x = fma(gev16(0), x1[1], conv_x);
+                conv_y = fma(gev(1), shyc, conv_y);
+                conv_z = fma(gev16(2), z3[1], conv_z);
+                const T hc2 = dif2(V(Sp, 1, 0, 0) + fvv(1), shyp, V(Sc, 1, 0, 0) + fvv(1), shyc);
+                const T d22 = mad3((T)MET(11), scjp, (T)MET(12), scc, (T)MET(13), scjm);
+                T cv = -(hc2 * rdyp);
+                cv = fma(-kz16, der24p(z3, w3), cv);
+                cv = fma(-kx16, der24p(x1, u1), cv);
+                const T convc = fma(svx, XL(Sc, 4), fma(svz, ZL(Sc, 4), cv));
+                o_rc[cz] = fma(tpG, convc, ttbs * d22);
                 o_hc[cz] = convc;
             }
+#undef XI
+#undef ZI
+#undef XL
+#undef ZL
 #undef V
 #undef MET
             o_rx[cz] = rhs_x; o_ry[cz] = rhs_y; o_rz[cz] = rhs_z;
@@ -508,15 +568,15 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
 #pragma unroll
             for (int cz = 0; cz < ZC; cz++) {
                 if (!act[cz]) continue;
-                const size_t q0 = q0a[cz];
-                fl.rx[q0] = (V)o_rx[cz];
-                fl.ry[q0] = (V)o_ry[cz];
-                fl.rz[q0] = (V)o_rz[cz];
+                const unsigned q0 = q0a[cz];
+                fl.rx[q0] = (V)fma(tpT, (T)hx0a[cz], o_rx[cz]);
+                fl.ry[q0] = (V)fma(tpT, (T)hy0a[cz], o_ry[cz]);
+                fl.rz[q0] = (V)fma(tpT, (T)hz0a[cz], o_rz[cz]);
                 fl.hx[q0] = (V)o_hx[cz];
                 fl.hy[q0] = (V)o_hy[cz];
                 fl.hz[q0] = (V)o_hz[cz];
                 if (SCALAR) {
-                    fl.rc[q0] = (V)o_rc[cz];
+                    fl.rc[q0] = (V)fma(tpT, (T)hc0a[cz], o_rc[cz]);
                     fl.hc[q0] = (V)o_hc[cz];
                 }
             }
@@ -535,7 +595,6 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
 #pragma unroll
                 for (int cz = 0; cz < ZC; cz++) { u64m[cz] = u64c[cz]; u64c[cz] = u64p[cz]; u64p[cz] = u64n[cz]; }
             }
-        __syncthreads();
             if constexpr (MULTI) {
                 // row j was work item tile*ny + j - 1: a logical block ends here
                 if ((long long)tile * ny + j == lb_end && lb + 1 < lb1) {
@@ -548,17 +607,25 @@ __device__ __forceinline__ void rhs_body(const G& grid, const DConst& c, const D
                 }
             }
         }
+        __syncthreads();  // the next tile's rows overwrite the ring
 #undef LOAD_ROW32
 #undef LOAD_ROW64
     }
     if constexpr (F64) cp_async_wait<0>();
 #undef KC
-#undef dxC
-#undef dzC
-#undef dxxC
-#undef dzzC
 #undef grav
 #undef gev
+#undef gev16
+#undef kx16
+#undef kz16
+#undef kx256
+#undef kz256
+#undef gx24
+#undef gz24
+#undef vx
+#undef vz
+#undef svx
+#undef svz
 #undef fvv
 
     // flow-rate constraint and the substep coefficients (last CTA)
@@ -644,10 +711,9 @@ __global__ void __launch_bounds__(RhsCfg<T, VAR>::NTHR, RhsCfg<T, VAR>::MINB)
 // ---------------------------------------------------------------------------
 // one wave of resident CTAs (MINB per SM for the precision; the record
 // count is sized for the larger)
+long long rhs_work_rows(const DConst& c) { return (long long)((c.nx + TX - 1) / TX) * ((c.nz + TZ - 1) / TZ) * c.ny; }
 static size_t rhs_blocks(const DConst& c, int minb) {
-    const long long rows = (long long)((c.nx + TX - 1) / TX) * ((c.nz + TZ - 1) / TZ) * c.ny;
-    const long long b = (long long)minb * (c.nsm > 0 ? c.nsm : 148);
-    return (size_t)(rows < b ? rows : b);
+    return (size_t)std::min<long long>(rhs_work_rows(c), (long long)minb * (c.nsm > 0 ? c.nsm : 148));
 }
 
 size_t rhs_grid_blocks(const DConst& c) {
@@ -714,8 +780,6 @@ void launch_rhs_tile(cudaStream_t st, const DConst& c, const DMetric& m, DCoef* 
 dim3 rhs_member_grid(const DConst& c, int f32arith) {
     return dim3((unsigned)rhs_blocks(c, f32arith ? RhsCfg<float, 0>::MINB : RhsCfg<double, 0>::MINB));
 }
-
-long long rhs_work_rows(const DConst& c) { return (long long)((c.nx + TX - 1) / TX) * ((c.nz + TZ - 1) / TZ) * c.ny; }
 
 int rhs_wave(const DConst& c) { return RhsCfg<double, 0>::MINB * (c.nsm > 0 ? c.nsm : 148); }
 
