@@ -276,7 +276,16 @@ __device__ __forceinline__ void helm_body(const G& grid, const DConst& cst, cons
         __syncwarp();
         V* const s = sd + lane;
         W f = 0;
+        // u is read on the way back: brought into L2 meanwhile
+        const V* pf = uc + (ptrdiff_t)jw * nx;
         for (int i0 = 0; i0 < nf; i0 += U) {
+            if (valid) {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(pf));
+                    pf += gstep;
+                }
+            }
             W g[U], mm[U];
 #pragma unroll
             for (int u = 0; u < U; u++) {
