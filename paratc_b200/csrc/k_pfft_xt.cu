@@ -706,14 +706,14 @@ bool xt_tma_supported(int n) {
 }
 
 void xt_tma_init() {
-#define X_CASE(n)                                                                                              \
-    cudaFuncSetAttribute(k_xb_tma<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);          \
-    cudaFuncSetAttribute(k_xb_tma32<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);        \
-    cudaFuncSetAttribute(k_xf_tma<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);       \
+#define X_CASE(n) \
+    cudaFuncSetAttribute(k_xb_tma<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem); \
+    cudaFuncSetAttribute(k_xb_tma32<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem); \
+    cudaFuncSetAttribute(k_xf_tma<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem); \
     cudaFuncSetAttribute(k_xb_tma_gather<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);\
     cudaFuncSetAttribute(k_xf_tma_scatter<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);\
-    cudaFuncSetAttribute(k_xf_div<n, double, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
-                         (int)XD<n>::smem);                                                                    \
+    cudaFuncSetAttribute(k_xf_div<n, double, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                         (int)XD<n>::smem); \
     cudaFuncSetAttribute(k_xf_div<n, float, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XD<n>::smem);
     XT_SIZES(X_CASE)
 #undef X_CASE
@@ -723,10 +723,10 @@ void launch_xb_tma(cudaStream_t st, int nx, int ny, int nz, const double2* spec,
                    const double2* post, double scale, int padded, int nsm, unsigned int* err) {
     const int nrows = ny * nz;
     switch (nx / 2) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        launch_pdl(k_xb_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, spec, \
-                   phi, twx, post, scale, padded, err);                                                        \
+#define X_CASE(n) \
+    case n: \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, spec, \
+                   phi, twx, post, scale, padded, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -738,10 +738,10 @@ void launch_xb_tma(cudaStream_t st, int nx, int ny, int nz, const float2* spec, 
                    const double2* post, double scale, int padded, int nsm, unsigned int* err) {
     const int nrows = ny * nz;
     switch (nx / 2) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        launch_pdl(k_xb_tma32<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny,   \
-                   spec, phi, twx, post, scale, padded, err);                                                  \
+#define X_CASE(n) \
+    case n: \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma32<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, \
+                   spec, phi, twx, post, scale, padded, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -753,10 +753,10 @@ void launch_xb_tma_gather(cudaStream_t st, int nx, int ny, int nz, const XtGathe
                           const double2* post, double scale, int nsm, unsigned int* err) {
     const int nrows = ny * nz;
     switch (nx / 2) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        launch_pdl(k_xb_tma_gather<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, \
-                   gt, phi, twx, post, scale, err);                                                            \
+#define X_CASE(n) \
+    case n: \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma_gather<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, \
+                   gt, phi, twx, post, scale, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -768,10 +768,10 @@ void launch_xf_tma_scatter(cudaStream_t st, int nx, int ny, int nz, const double
                            const double2* twx, const double2* post, int nsm, unsigned int* err) {
     const int nrows = ny * nz;
     switch (nx / 2) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        launch_pdl(k_xf_tma_scatter<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows,   \
-                   ny, src, gt, twx, post, err);                                                               \
+#define X_CASE(n) \
+    case n: \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xf_tma_scatter<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, \
+                   ny, src, gt, twx, post, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -783,10 +783,10 @@ void launch_xf_tma(cudaStream_t st, int nx, int ny, int nz, const double* src, d
                    const double2* post, int nsm, unsigned int* err) {
     const int nrows = ny * nz;
     switch (nx / 2) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        launch_pdl(k_xf_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, src, spec, \
-                   twx, post, err);                                                                            \
+#define X_CASE(n) \
+    case n: \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xf_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, src, spec, \
+                   twx, post, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -815,10 +815,10 @@ static void xf_div_t(cudaStream_t st, int mode, const DConst& c, const DMetric& 
     const int nrows = c.ny * c.nz;
     const int grid = xf_div_grid(c.nx / 2, nrows, c.nsm > 0 ? c.nsm : 148);
     switch (c.nx / 2) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        launch_pdl(k_xf_div<n, V, S>, dim3(grid), dim3(XD<n>::NT), XD<n>::smem, st, mode, c, m, coef, f.ux, f.uy, \
-                   f.uz, spec, twx, post, part, counter, out_max, err);                                        \
+#define X_CASE(n) \
+    case n: \
+        launch_pdl_if(pdl_pays((size_t)c.nx * c.ny * c.nz), k_xf_div<n, V, S>, dim3(grid), dim3(XD<n>::NT), XD<n>::smem, st, mode, c, m, coef, f.ux, f.uy, \
+                   f.uz, spec, twx, post, part, counter, out_max, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE

@@ -161,8 +161,8 @@ static void pfft_z_t(cudaStream_t st, int dir, int nx, int ny, int nz, S* spec, 
     case n: {                                                                                                     \
         const int grid = (ncol + ZK<n, A>::B - 1) / ZK<n, A>::B;                                                  \
         if (dir < 0)                                                                                              \
-            launch_pdl(k_zt<n, -1, S, A>, dim3(grid), dim3(ZK<n, A>::P), ZK<n, A>::smem, st, ncol, spec, twz);    \
-        else launch_pdl(k_zt<n, 1, S, A>, dim3(grid), dim3(ZK<n, A>::P), ZK<n, A>::smem, st, ncol, spec, twz);    \
+            launch_pdl_if(pdl_pays((size_t)2 * ncol * n), k_zt<n, -1, S, A>, dim3(grid), dim3(ZK<n, A>::P), ZK<n, A>::smem, st, ncol, spec, twz);    \
+        else launch_pdl_if(pdl_pays((size_t)2 * ncol * n), k_zt<n, 1, S, A>, dim3(grid), dim3(ZK<n, A>::P), ZK<n, A>::smem, st, ncol, spec, twz);    \
         break;                                                                                                    \
     }
         PFFT_Z_SIZES(Z_CASE)

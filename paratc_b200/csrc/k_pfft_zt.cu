@@ -205,8 +205,9 @@ static void zt_tma_t(cudaStream_t st, int dir, int ncol, int nz, const void* tma
         const int per_sm = (int)((220 * 1024) / Z::smem);                                                      \
         int grid = (per_sm > 0 ? per_sm : 1) * nsm;                                                            \
         if (grid > nb) grid = nb;                                                                              \
-        if (dir < 0) launch_pdl(k_zt_tma<n, -1, w, A>, dim3(grid), dim3(Z::P), Z::smem, st, tm, nb, twz, err);  \
-        else launch_pdl(k_zt_tma<n, 1, w, A>, dim3(grid), dim3(Z::P), Z::smem, st, tm, nb, twz, err);           \
+        const bool early = pdl_pays((size_t)2 * ncol * nz); \
+        if (dir < 0) launch_pdl_if(early, k_zt_tma<n, -1, w, A>, dim3(grid), dim3(Z::P), Z::smem, st, tm, nb, twz, err);  \
+        else launch_pdl_if(early, k_zt_tma<n, 1, w, A>, dim3(grid), dim3(Z::P), Z::smem, st, tm, nb, twz, err);           \
     }
     if (zt_wide(ncol, nz, (int)sizeof(A))) {
         if (nz == 512) ZT_LAUNCH(512, 1)

@@ -664,12 +664,13 @@ static dim3 project_grid(const DConst& c) {
 template <class V>
 static void project_t(cudaStream_t st, const DConst& c, const DMetric& m, const DCoef* coef, int mode, const V* phi,
                       const FieldSet<V>& f, const double* uy_ym) {
+    const bool early = pdl_pays((size_t)c.nx * c.ny * c.nz);
     if (c.nx % 2 == 0)
-        launch_pdl(k_project2<V>, dim3((c.nx + 63) / 64, (c.ny + 7) / 8, c.nz), cell_block(), 0, st, c, m, coef, mode,
-                   phi, f.ux, f.uy, f.uz, f.pr, uy_ym);
+        launch_pdl_if(early, k_project2<V>, dim3((c.nx + 63) / 64, (c.ny + 7) / 8, c.nz), cell_block(), 0, st, c, m,
+                      coef, mode, phi, f.ux, f.uy, f.uz, f.pr, uy_ym);
     else
-        launch_pdl(k_project<V>, project_grid(c), cell_block(), 0, st, c, m, coef, mode, phi, f.ux, f.uy, f.uz, f.pr,
-                   uy_ym);
+        launch_pdl_if(early, k_project<V>, project_grid(c), cell_block(), 0, st, c, m, coef, mode, phi, f.ux, f.uy,
+                      f.uz, f.pr, uy_ym);
 }
 void launch_project(cudaStream_t st, const DConst& c, const DMetric& m, const DCoef* coef, int mode, const double* phi,
                     const Fields& f, const double* uy_ym) {

@@ -12,9 +12,10 @@ bool pdl_enabled();
 // launch with programmatic stream serialization, so that the kernel's CTAs
 // can be scheduled while the previous kernel in the stream drains; the
 // kernel itself calls pdl_wait() before touching data of earlier kernels
+// (early = false: an ordinary launch)
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                       Args&&... args) {
+inline void launch_pdl_if(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                          Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -24,9 +25,27 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = early && pdl_enabled() ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
+template <typename... KArgs, typename... Args>
+inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                       Args&&... args) {
+    launch_pdl_if(true, kernel, grid, block, smem, st, std::forward<Args>(args)...);
+}
+
+// Whether the transforms and the projection of a grid of `cells` start early.
+// A small grid's launch latency is worth hiding; on a large one the waiting
+// CTAs take shared memory and L1 from the kernel that still runs, and keep an
+// SM's shared-memory split where that kernel set it (the projection, which
+// lives from L1, follows the inverse transform, which takes all of the shared
+// memory).  One B200, early against ordinary launch of these kernels: step of
+// 128 x 96 x 128 0.482 against 0.497 ms, of 384 x 192 x 256 5.24 against 4.96
+// ms, of 1536 x 160 x 256 21.7 against 21.1 ms; Poisson solve of 512 x 256 x
+// 512 1190 against 1102 us.  In between: 1.021 against 1.003 ms at 192 x 96 x
+// 192, 1.267 against 1.274 at 256 x 128 x 128, 1.81 against 1.80 at 256 x 128
+// x 192.
+inline bool pdl_pays(size_t cells) { return cells <= ((size_t)3 << 20); }
 
 // device pointers of the fields of one context (padded layout, see
 // common.cuh), in storage type V: double for the FP64 forms, float for the
