@@ -69,6 +69,7 @@ struct paratc_ctx {
     bool ztma_ok = false;  // its tensor map is encoded (nz supported, driver entry point found)
     bool xtma = false;     // x transforms through the bulk-copy-fed persistent kernels (split path)
     bool xdiv = false;     // the divergence source by producer warps of the forward x transform
+    bool sched_auto = true;  // the schedule is default_schedule's, not the caller's
     alignas(64) unsigned char zt_tmap[128];  // its tensor map (a CUtensorMap)
     alignas(64) unsigned char zt_tmap32[128];  // the same over the float2 spectrum of the FP32 storage form
     bool ztma32_ok = false;                    // that map is encoded (ncol even, nz supported)
@@ -118,6 +119,7 @@ static std::string tune_key(const paratc_ctx* ctx);
 static bool tune_cache_read(const char* path, const std::string& key, paratc_tuning* t);
 static bool tuning_valid(const paratc_ctx* ctx, const paratc_tuning& t);
 static void tuning_apply(paratc_ctx* ctx, const paratc_tuning& t);
+static void default_schedule(paratc_ctx* ctx);
 
 namespace {
 
@@ -680,8 +682,6 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
         return PARATC_ERR_BAD_ARG;
     }
     ctx->pfft = pfft_x_supported(ctx->nx / 2) && pfft_z_supported(ctx->nz) && std::getenv("PARATC_GENERIC_FFT") == nullptr;
-    // PARATC_NO_PLANE keeps the separate x and z transform kernels (both exact)
-    ctx->plane = ctx->pfft && plane_supported(ctx->nx, ctx->nz) && std::getenv("PARATC_NO_PLANE") == nullptr;
     cudaError_t ce = cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking);
     if (ce != cudaSuccess) { delete ctx; return PARATC_ERR_CUDA; }
     // the kernels' shared-memory limits are attributes of each device: set
@@ -758,7 +758,7 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
     // k_cfl, one per block of the RHS and forward-x kernels, 8 per block of the
     // end-of-step kernel
     ctx->npart = std::max(std::max(4 * cell_grid_blocks(kc), rhs_grid_blocks(kc)),
-                          std::max((size_t)pfft_x_blocks(ctx->nx, ctx->ny, ctx->nz), endstep_blocks(kc) * 8)) + 64;
+                          std::max((size_t)pfft_x_blocks(ctx->nx, ctx->ny, ctx->nz), endstep_blocks(kc) * 8)) + 64 + 3 * (size_t)kc.nsm;
     if ((rc = dalloc(ctx, &ctx->d_src, ctx->ni)) || (rc = dalloc(ctx, &ctx->d_spec, (size_t)ctx->M1 * ctx->ny * ctx->nz)) ||
         (rc = dalloc(ctx, &ctx->d_part, ctx->npart)) || (rc = dalloc(ctx, &ctx->d_uy_ym, (size_t)ctx->nx * ctx->nz)) ||
         (rc = dalloc(ctx, &ctx->d_duy_ym, (size_t)ctx->nx * ctx->nz)) || (rc = dalloc(ctx, &ctx->d_coef, 1)) ||
@@ -810,16 +810,16 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(ctx->st));
     }
-    // z transforms fed by TMA: the default of the separate-transform path
-    // where nz has a kernel; PARATC_ZT_TMA=0 keeps the register-fed k_zt
+    // PARATC_NO_PLANE keeps the separate x and z transform kernels,
+    // PARATC_ZT_TMA=0 the register-fed k_zt, PARATC_XT_TMA=0 the register-fed
+    // x kernels (all exact)
     if (ctx->pfft && zt_tma_supported(ctx->nz))
         ctx->ztma_ok = zt_tma_prepare(ctx->d_spec, ctx->ny * (ctx->nx / 2 + 1), ctx->nz, ctx->zt_tmap);
     {
-        const char* e = std::getenv("PARATC_ZT_TMA");
-        ctx->ztma = ctx->ztma_ok && !ctx->plane && !(e && std::atoi(e) == 0);
         const char* ex = std::getenv("PARATC_XT_TMA");
         ctx->xtma = ctx->pfft && xt_tma_supported(ctx->nx / 2) && !(ex && std::atoi(ex) == 0);
     }
+    default_schedule(ctx);
     // twiddles
     {
         std::vector<double2> twx = twiddles(ctx->nx / 2, ctx->nx / 2);
@@ -1144,7 +1144,33 @@ static bool sched_supported(const paratc_ctx* ctx, int choice) {
     return true;
 }
 
+extern "C++" {
+// The schedule of a context whose caller picks none, by the grid and the
+// storage form.
+//  - One CTA per y plane where the planes are so small that two CTAs share an
+//    SM; with one (128 x 128 planes) the separate transforms win.  One B200,
+//    fused against separate: 37 / 49 us per solve of 96 x 96 x 96, 33 / 44 of
+//    64 x 96 x 128, 53 / 50 of 128 x 96 x 128.
+//  - Else the divergence by the producers of the forward x transform, against
+//    computing it in the transform: 73 / 90 us at 192 x 96 x 128, 459 / 518
+//    at 384 x 192 x 256, 1.44 / 1.90 ms at 1536 x 160 x 256.  Rows too long
+//    for the marching producers (nx > 1536) gain in FP64 only (0.97 / 1.27 ms
+//    at 2304 x 64 x 192, 0.79 / 0.67 in the FP32 form).
+//  - z by TMA where nz has the kernel, unless the spectrum's planes are far
+//    apart and short, so that a batch meets a page per row: 1.44 ms with the
+//    register-fed z at 1536 x 160 x 256 (2 MB), 1.55 with TMA.
+static void default_schedule(paratc_ctx* ctx) {
+    const auto off = [](const char* name) { const char* e = std::getenv(name); return e && std::atoi(e) == 0; };
+    ctx->plane = ctx->pfft && plane_supported(ctx->nx, ctx->nz) && plane_smem(ctx->nx, ctx->nz) <= 110 * 1024 &&
+                 std::getenv("PARATC_NO_PLANE") == nullptr;
+    const size_t apart = (size_t)ctx->ny * ctx->M1 * sizeof(double2);
+    ctx->ztma = ctx->ztma_ok && !ctx->plane && !off("PARATC_ZT_TMA") && !(ctx->nz <= 256 && apart > ((size_t)1 << 20));
+    ctx->xdiv = ctx->xtma && !ctx->plane && (ctx->prec != PARATC_PREC_FP32 || xf_div_marches(ctx->nx / 2));
+}
+}  // extern "C++"
+
 static void sched_apply(paratc_ctx* ctx, int choice) {
+    ctx->sched_auto = false;
     const int sc = choice / 2;
     ctx->plane = sc == 0;
     ctx->pfft = sc == 0 || sc == 1 || sc >= 3;
@@ -1194,6 +1220,7 @@ int paratc_set_precision(paratc_ctx* ctx, int prec) {
         state_to64(ctx);
     }
     ctx->prec = prec;
+    if (ctx->sched_auto) default_schedule(ctx);
     ctx->kc.fp32_rhs = prec == PARATC_PREC_MIXED ? 1 : 0;
     ctx->next_ready = false;  // the next step takes its CFL from the converted state
     ctx->sched_gen++;         // captured graphs hold the other kernels

@@ -80,4 +80,131 @@ __device__ __forceinline__ void div_batch(const DConst& c, const DMetric& m, con
     }
 }
 
+// The same sources with a thread marching through k: it owns NPT point pairs
+// (e0, e0 + Q, ...) of one row jc and, plane by plane, takes one new pair of w
+// (the other three taps stay in registers), u01 and the two v pairs; the x
+// neighbours of u01 come from the neighbouring lanes.  So a pair of points
+// costs four 16-byte loads instead of nine.  They go to slots of the thread's
+// own in shared memory (cp.async, D planes ahead, no barrier), which keeps
+// more of them in flight than registers could: the nine-load form was bound
+// by that.
+template <class V>
+struct MarchPair;
+template <>
+struct MarchPair<double> {
+    using T = double2;
+};
+template <>
+struct MarchPair<float> {
+    using T = float2;
+};
+template <int BYTES>
+__device__ __forceinline__ void march_copy(void* sdst, const void* gsrc) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
+}
+
+// planes k0 .. k1-1 of row j (0-based; on: the thread has a pair and its row
+// lies inside the grid); ring: [D][NPT][4][Q] pairs.  begin(k) runs before
+// plane k's values are stored, st(k, e, value) stores them, done(k) runs after
+// them; all threads of the group take every step.  begin returns false to stop.
+template <int N, int Q, int NPT, int D, class V, class BEG, class ST, class DONE>
+__device__ __forceinline__ bool div_march(const DConst& c, const DMetric& m, const V* __restrict__ ux,
+                                          const V* __restrict__ uy, const V* __restrict__ uz, int j, int e0, bool on,
+                                          int k0, int k1, double sudtal, double& dm,
+                                          typename MarchPair<V>::T* __restrict__ ring, int tp, const BEG& begin,
+                                          const ST& st, const DONE& done) {
+    using P2 = typename MarchPair<V>::T;
+    const int nx = c.nx, nz = c.nz, lane = threadIdx.x & 31;
+    const unsigned pl = (unsigned)c.nyt * nx, r0 = (unsigned)(on ? j + 1 : 1) * nx, off = r0 + 2 * e0;
+    const double rdyp = on ? __ldg(&m.rdyp[j + 1]) : 0.0;
+    auto pair = [](const V* p) { return __ldg(reinterpret_cast<const P2*>(p)); };
+    auto has = [&](int p) { return N % Q == 0 || p + 1 < NPT || e0 + p * Q < N; };
+    auto el = [&](int p) { return lane == 0 || e0 + p * Q == 0; };
+    auto er = [&](int p) { return lane == 31 || e0 + p * Q == N - 1; };
+    auto plane = [&](int k) { return (unsigned)(k < 0 ? k + nz : (k >= nz ? k - nz : k)) * pl; };
+    P2* const my = ring + tp;
+    auto copy = [&](int k, int d) {  // plane k's pairs into ring slot d
+        const unsigned a = (unsigned)k * pl;
+        const V *ru = ux + a + off, *rv = uy + a + off, *rw = uz + plane(k + 2) + off;
+#pragma unroll
+        for (int p = 0; p < NPT; p++) {
+            if (!on || !has(p)) continue;
+            P2* s = my + (d * NPT + p) * 4 * Q;
+            march_copy<sizeof(P2)>(s, ru + 2 * p * Q);
+            march_copy<sizeof(P2)>(s + Q, rv + 2 * p * Q);
+            march_copy<sizeof(P2)>(s + 2 * Q, rv + 2 * p * Q + nx);
+            march_copy<sizeof(P2)>(s + 3 * Q, rw + 2 * p * Q);
+        }
+    };
+    P2 w[3][NPT], ur[NPT];
+    V ul[NPT];
+    auto edges = [&](int k) {  // the neighbours that no lane of the warp holds
+        const V* ru = ux + (unsigned)k * pl + off;
+#pragma unroll
+        for (int p = 0; p < NPT; p++) {
+            if (!on || !has(p)) continue;
+            if (el(p)) ul[p] = __ldg(e0 + p * Q == 0 ? ru + nx - 1 : ru + 2 * p * Q - 1);
+            if (er(p)) ur[p] = pair(e0 + p * Q == N - 1 ? ru + 2 * p * Q + 2 - nx : ru + 2 * p * Q + 2);
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+#pragma unroll
+        for (int p = 0; p < NPT; p++)
+            if (on && has(p)) w[q][p] = pair(uz + plane(k0 - 1 + q) + off + 2 * p * Q);
+    for (int d = 0; d < D; d++) {
+        if (k0 + d < k1) copy(k0 + d, d);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    edges(k0);
+    int d = 0;
+    for (int k = k0; k < k1; k++) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
+        double2 val[NPT];
+#pragma unroll
+        for (int p = 0; p < NPT; p++) {
+            const P2* s = my + (d * NPT + p) * 4 * Q;
+            const P2 u01 = s[0], v0 = s[Q], v1 = s[2 * Q], w3 = s[3 * Q];
+            // (lanes without a pair take part in the exchange)
+            const V lx = __shfl_up_sync(0xffffffffu, u01.y, 1);
+            const V rx = __shfl_down_sync(0xffffffffu, u01.x, 1);
+            const V ry = __shfl_down_sync(0xffffffffu, u01.y, 1);
+            DivTaps q;
+            q.u01 = make_double2(u01.x, u01.y);
+            q.um = el(p) ? ul[p] : lx;
+            q.u23 = er(p) ? make_double2(ur[p].x, ur[p].y) : make_double2(rx, ry);
+            q.v0 = make_double2(v0.x, v0.y);
+            q.v1 = make_double2(v1.x, v1.y);
+            q.w0 = make_double2(w[0][p].x, w[0][p].y);
+            q.w1 = make_double2(w[1][p].x, w[1][p].y);
+            q.w2 = make_double2(w[2][p].x, w[2][p].y);
+            q.w3 = make_double2(w3.x, w3.y);
+            q.rdyp = rdyp;
+            const double2 dv = div_eval(q, c);
+            const bool act = on && has(p);
+            if (act) dm = nmax(dm, nmax(fabs(dv.x), fabs(dv.y)));
+            val[p] = act ? make_double2(sudtal * dv.x, sudtal * dv.y) : make_double2(0.0, 0.0);
+            w[0][p] = w[1][p];
+            w[1][p] = w[2][p];
+            w[2][p] = w3;
+        }
+        if (k + 1 < k1) edges(k + 1);
+        if (k + D < k1) copy(k + D, d);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        d = d + 1 == D ? 0 : d + 1;
+        if (!begin(k)) {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            return false;
+        }
+#pragma unroll
+        for (int p = 0; p < NPT; p++)
+            if (has(p)) st(k, e0 + p * Q, val[p]);
+        done(k);
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    return true;
+}
+
 }  // namespace ptc

@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
 // ---------------------------------------------------------------------------
 // Forward transform of the divergence source (clcPrSrc, src/m_TScheme.f90:
 // 48-77: scaled by 1/pmAlpha in mode 0, unscaled in mode 1, max|div| reduced
-// over the grid by the last CTA), warp-specialised: XD_Q producer threads
+// over the grid by the last CTA), warp-specialised: XD::Q producer threads
 // compute the divergence of the next batch's rows from u, v, w into one
 // stage while the P consumer threads transform the other stage, split it
 // into the nx/2+1 modes and send the spectrum rows out by bulk stores.
@@ -510,9 +510,17 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
 // that reduces the predicate, so all its threads decide alike.  Every wait is
 // bounded; a group that gives up leaves its loop, the other group's waits
 // then run out too, and the CTA records *err |= 4.
+//
+// The producers march through k (div_march, div_src.cuh), so a batch is KB
+// planes of JB rows and a CTA takes a contiguous range of batches in k-fastest
+// order.  The transform by the same threads that compute the divergence (k_xf)
+// waits for nine loads per pair of points with few of them in flight.  One
+// B200, divergence and transform, k_xf against this kernel: 258 / 172 us at
+// 384 x 192 x 256, 1.06 / 0.63 ms at 1536 x 160 x 256 (0.31 ms of memory at
+// the copy rate; there the 192 transforming threads of an SM set the pace),
+// 28 / 27 us at 128 x 96 x 128.
 // ---------------------------------------------------------------------------
-constexpr int XD_Q = 256;      // producer threads
-constexpr int XD_DIV_U = 2;    // divergence point pairs in flight per producer thread
+constexpr int XD_DIV_U = 2;    // point pairs in flight per producer thread where it does not march (XD::MARCH)
 
 template <int N>
 struct XD {
@@ -534,8 +542,39 @@ struct XD {
     }
     static constexpr int PITCH = pitch();
     static constexpr unsigned STAGE = (unsigned)B * PITCH;
-    static constexpr int NT = P + XD_Q;
-    static constexpr size_t smem = 2 * (size_t)STAGE * sizeof(double2);
+    // Producers: they march through k (div_march) where a thread's pairs fit
+    // its registers; the longest rows keep the nine-load form
+    static constexpr bool MARCH = N <= 768;
+    // (a multiple or a divisor of the row's pairs, so that none idles)
+    static constexpr int Q = !MARCH ? 256
+                             : N % 5 == 0 ? 160
+                             : N % 3 == 0 ? (N <= 48 ? 96 : N <= 192 ? 192 : 384)
+                                          : (N <= 64 ? 128 : 256);
+    static constexpr int NT = P + Q;
+    // a batch is JB rows jc of KB planes k: row b is plane b / JB, row b % JB
+    static constexpr int pow2(int v) { return v >= 2 ? 2 * pow2(v / 2) : 1; }
+    static constexpr int jcalc() {
+        const int j = N >= Q ? 1 : pow2(Q / N);
+        return !MARCH || j > B ? B : j;
+    }
+    static constexpr int JB = jcalc(), KB = B / JB;
+    static_assert(B % JB == 0, "a batch is whole planes");
+    static constexpr int NPT = N >= Q ? (N + Q - 1) / Q : 1;  // pairs per marching thread
+    // CTAs per SM: more where the rows are short
+    static constexpr int MINB(int vsize) { return N <= 64 && vsize == 4 ? 3 : (N <= 256 ? 2 : 1); }
+    // shared memory (vsize: bytes of a stored value): the two stages (with
+    // the float2 twiddles after them in the FP32 form), then D planes of the
+    // producers' pairs
+    static constexpr size_t base(int vsize) {
+        return (2 * (size_t)STAGE * 2 * vsize + (vsize == 4 ? (size_t)N * 2 * vsize : 0) + 127) / 128 * 128;
+    }
+    static constexpr size_t plane(int vsize) { return MARCH ? (size_t)NPT * Q * 4 * 2 * vsize : 0; }
+    static constexpr int D(int vsize) {
+        if (!MARCH) return 0;
+        const int d = (int)(((size_t)(MINB(vsize) == 3 ? 70 : MINB(vsize) == 2 ? 108 : 220) * 1024 - base(vsize)) / plane(vsize));
+        return d < 1 ? 1 : (d > 6 ? 6 : d);
+    }
+    static constexpr size_t smem(int vsize) { return base(vsize) + D(vsize) * plane(vsize); }
 };
 
 // V: storage of the velocity, S: of the spectrum.  The FP32 storage form
@@ -543,12 +582,12 @@ struct XD {
 // stores: a float2 row of N+1 values starts 16-byte aligned only at even
 // rows, which a bulk store needs.
 template <int N, class V, class S>
-__global__ void __launch_bounds__(XD<N>::NT, 1)
+__global__ void __launch_bounds__(XD<N>::NT, XD<N>::MINB(sizeof(V)))
     k_xf_div(int mode, DConst c, DMetric m, const DCoef* __restrict__ coef, const V* __restrict__ ux,
              const V* __restrict__ uy, const V* __restrict__ uz, S* __restrict__ spec,
              const double2* __restrict__ twN, const double2* __restrict__ post, double* __restrict__ part,
              unsigned int* __restrict__ counter, double* __restrict__ out_max, unsigned int* __restrict__ err) {
-    constexpr int B = XD<N>::B, P = XD<N>::P, PITCH = XD<N>::PITCH, M1 = N + 1, Q = XD_Q;
+    constexpr int B = XD<N>::B, P = XD<N>::P, PITCH = XD<N>::PITCH, M1 = N + 1, Q = XD<N>::Q;
     static_assert(P % 32 == 0, "the consumer group is whole warps");
     // the passes' complex type: float2 for the FP32 storage form (the stages
     // hold float2, half the FP64 stage, and the float2 twiddles sit after
@@ -556,22 +595,33 @@ __global__ void __launch_bounds__(XD<N>::NT, 1)
     using A = std::conditional_t<sizeof(S) == sizeof(float2), float2, double2>;
     constexpr bool F32 = sizeof(A) == sizeof(float2);
     constexpr unsigned SB = XD<N>::STAGE;
-    static_assert(!F32 || 2 * SB >= (unsigned)N, "the twiddles fit after the float2 stages");
     constexpr ff::Sched SC = ff::make_sched(N);
     extern __shared__ __align__(128) unsigned char smraw[];
     A* stage[2] = {reinterpret_cast<A*>(smraw), reinterpret_cast<A*>(smraw) + SB};
-    float2* tws32 = reinterpret_cast<float2*>(smraw) + 2 * SB;
+    A* tws = stage[0] + 2 * SB;
+    auto* ring = reinterpret_cast<typename MarchPair<V>::T*>(smraw + XD<N>::base(sizeof(V)));
     __shared__ unsigned long long full[2], empty[2];
     __shared__ int bad_c, bad_p;
     const int tid = threadIdx.x;
-    const int nrows = c.ny * c.nz;
-    const int nb = (nrows + B - 1) / B;
+    constexpr int JB = XD<N>::JB, KB = XD<N>::KB;
+    const int ny = c.ny, nz = c.nz;
+    // batches in k-fastest order; a CTA takes a contiguous range of them
+    const int nbk = (nz + KB - 1) / KB, nb = (ny + JB - 1) / JB * nbk;
+    const int bt0 = (int)((long long)nb * blockIdx.x / gridDim.x);
+    const int bt1 = (int)((long long)nb * (blockIdx.x + 1) / gridDim.x);
+    // spectrum row of batch row b (-1: outside the grid)
+    auto row_of = [&](int bt, int b) {
+        const int jb = bt / nbk, j = jb * JB + b % JB, k = (bt - jb * nbk) * KB + b / JB;
+        return j < ny && k < nz ? k * ny + j : -1;
+    };
     const long long lim = tma::wait_limit(err);
-    if constexpr (F32)
-        for (int t = tid; t < N; t += XD<N>::NT) tws32[t] = cto<float2>(twN[t]);
     const A* tw;
-    if constexpr (F32) tw = reinterpret_cast<const A*>(tws32);
-    else tw = reinterpret_cast<const A*>(twN);
+    if constexpr (F32) {
+        for (int t = tid; t < N; t += XD<N>::NT) tws[t] = cto<A>(twN[t]);
+        tw = tws;
+    } else {
+        tw = reinterpret_cast<const A*>(twN);
+    }
     if (tid == 0) {
         tma::mbar_init(&full[0], Q);
         tma::mbar_init(&full[1], Q);
@@ -588,23 +638,54 @@ __global__ void __launch_bounds__(XD<N>::NT, 1)
         // producers
         const int tp = tid - P;
         const double sudtal = (mode == 0) ? 1.0 / coef->pmAlpha : 1.0;
-        int it = 0;
-        for (int bt = blockIdx.x; bt < nb; bt += gridDim.x, it++) {
-            const int s = it & 1;
-            const bool ok = it < 2 || tma::mbar_wait(&empty[s], (unsigned)(((it >> 1) + 1) & 1), lim);
-            if (ff::group_any<2, Q>(!ok)) {
+        if constexpr (!XD<N>::MARCH) {
+            for (int bt = bt0; bt < bt1; bt++) {
+                const int it = bt - bt0, sg = it & 1, jb = bt / nbk, k = bt - jb * nbk;
+                const bool ok = it < 2 || tma::mbar_wait(&empty[sg], (unsigned)(((it >> 1) + 1) & 1), lim);
+                if (ff::group_any<2, Q>(!ok)) {
+                    bad_p = 1;
+                    break;
+                }
+                A* buf = stage[sg];
+                div_batch<N, B, Q, XD_DIV_U>(c, m, ux, uy, uz, k * ny + jb * JB, (k + 1) * ny, sudtal, tp, dm,
+                                             [&](int b, int e, double2 v) { buf[b * PITCH + e] = cto<A>(v); });
+                tma::mbar_arrive(&full[sg]);
+            }
+        } else {
+        const int jj = N >= Q ? 0 : tp / N, e0 = N >= Q ? tp : tp - jj * N;
+        for (int bt = bt0; bt < bt1;) {
+            // the batches of one row block: planes k0 .. k1-1
+            const int jb = bt / nbk, be = min(bt1, (jb + 1) * nbk);
+            const int k0 = (bt - jb * nbk) * KB, k1 = min(nz, (be - jb * nbk) * KB);
+            const bool mine = jj < JB && jb * JB + jj < ny;
+            A* buf = nullptr;
+            const bool ok = div_march<N, Q, XD<N>::NPT, XD<N>::D(sizeof(V))>(
+                c, m, ux, uy, uz, jb * JB + jj, e0, mine, k0, k1, sudtal, dm, ring, tp,
+                [&](int k) {
+                    if ((k - k0) % KB) return true;
+                    // a new batch: its stage must be free
+                    const int it = bt + (k - k0) / KB - bt0, sg = it & 1;
+                    buf = stage[sg];
+                    const bool free = it < 2 || tma::mbar_wait(&empty[sg], (unsigned)(((it >> 1) + 1) & 1), lim);
+                    return !ff::group_any<2, Q>(!free);
+                },
+                [&](int k, int e, double2 v) {
+                    if (jj < JB) buf[((k - k0) % KB * JB + jj) * PITCH + e] = cto<A>(v);
+                },
+                [&](int k) {
+                    if ((k - k0) % KB == KB - 1 || k == nz - 1) tma::mbar_arrive(&full[(bt + (k - k0) / KB - bt0) & 1]);
+                });
+            if (!ok) {
                 bad_p = 1;
                 break;
             }
-            A* buf = stage[s];
-            div_batch<N, B, Q, XD_DIV_U>(c, m, ux, uy, uz, bt * B, nrows, sudtal, tp, dm,
-                                         [&](int b, int e, double2 v) { buf[b * PITCH + e] = cto<A>(v); });
-            tma::mbar_arrive(&full[s]);
+            bt = be;
+        }
         }
     } else {
         // consumers
         int it = 0;
-        for (int bt = blockIdx.x; bt < nb; bt += gridDim.x, it++) {
+        for (int bt = bt0; bt < bt1; bt++, it++) {
             const int s = it & 1;
             A* buf = stage[s];
             if (ff::group_any<1, P>(!tma::mbar_wait(&full[s], (unsigned)((it >> 1) & 1), lim))) {
@@ -615,12 +696,12 @@ __global__ void __launch_bounds__(XD<N>::NT, 1)
             if constexpr (sizeof(S) != sizeof(double2)) {
                 // the split straight to the float2 spectrum rows (consecutive
                 // threads take consecutive modes of one row: coalesced stores)
-                const int g0 = bt * B, nv = min(B, nrows - g0);
-                for (int f = tid; f < nv * (N / 2 + 1); f += P) {
+                for (int f = tid; f < B * (N / 2 + 1); f += P) {
                     const int b = f / (N / 2 + 1), a = f - b * (N / 2 + 1);
-                    const int bn = N - a;
+                    const int bn = N - a, g = row_of(bt, b);
+                    if (g < 0) continue;
                     const A* rb = buf + b * PITCH;
-                    S* out = spec + (size_t)(g0 + b) * M1;
+                    S* out = spec + (size_t)g * M1;
                     const A za = rb[a], zb = rb[a == 0 ? 0 : bn];
                     const float h = 0.5f;
                     const A E = Cx<A>::make(h * (za.x + zb.x), h * (za.y - zb.y));
@@ -660,10 +741,12 @@ __global__ void __launch_bounds__(XD<N>::NT, 1)
             tma::fence_async_smem();
             ff::group_sync<1, P>();
             if (tid == 0) {
-                const int g0 = bt * B, nv = min(B, nrows - g0);
-                for (int b = 0; b < nv; b++)
-                    tma::bulk_store(reinterpret_cast<double2*>(spec) + (size_t)(g0 + b) * M1, buf + b * PITCH,
-                                    M1 * (unsigned)sizeof(double2));
+                for (int b = 0; b < B; b++) {
+                    const int g = row_of(bt, b);
+                    if (g >= 0)
+                        tma::bulk_store(reinterpret_cast<double2*>(spec) + (size_t)g * M1, buf + b * PITCH,
+                                        M1 * (unsigned)sizeof(double2));
+                }
                 tma::bulk_commit();
                 tma::bulk_wait_read0();  // the stores have read the stage
                 tma::mbar_arrive(&empty[s]);
@@ -713,8 +796,9 @@ void xt_tma_init() {
     cudaFuncSetAttribute(k_xb_tma_gather<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);\
     cudaFuncSetAttribute(k_xf_tma_scatter<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);\
     cudaFuncSetAttribute(k_xf_div<n, double, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                         (int)XD<n>::smem); \
-    cudaFuncSetAttribute(k_xf_div<n, float, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XD<n>::smem);
+                         (int)XD<n>::smem(8)); \
+    cudaFuncSetAttribute(k_xf_div<n, float, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                         (int)XD<n>::smem(4));
     XT_SIZES(X_CASE)
 #undef X_CASE
 }
@@ -794,31 +878,41 @@ void launch_xf_tma(cudaStream_t st, int nx, int ny, int nz, const double* src, d
     }
 }
 
-// one CTA per SM (the producers' loads and the consumers' transforms share
-// it), at most one batch per CTA
-int xf_div_grid(int n, int nrows, int nsm) {
-    int b = 1;
+// XD::MINB CTAs per SM (the producers' loads and the consumers' transforms
+// share it), at least one batch per CTA
+int xf_div_grid(int n, int ny, int nz, int nsm, int vsize) {
     switch (n) {
-#define X_CASE(n) case n: b = XD<n>::B; break;
+#define X_CASE(n) \
+    case n: { \
+        const int nb = (ny + XD<n>::JB - 1) / XD<n>::JB * ((nz + XD<n>::KB - 1) / XD<n>::KB); \
+        return nb < XD<n>::MINB(vsize) * nsm ? nb : XD<n>::MINB(vsize) * nsm; \
+    }
         XT_SIZES(X_CASE)
 #undef X_CASE
-        default: break;
+        default: return 1;
     }
-    const int nb = (nrows + b - 1) / b;
-    return nb < nsm ? nb : nsm;
+}
+
+bool xf_div_marches(int n) {
+    switch (n) {
+#define X_CASE(n) case n: return XD<n>::MARCH;
+        XT_SIZES(X_CASE)
+#undef X_CASE
+        default: return false;
+    }
 }
 
 template <class V, class S>
 static void xf_div_t(cudaStream_t st, int mode, const DConst& c, const DMetric& m, const DCoef* coef,
                      const FieldSet<V>& f, S* spec, const double2* twx, const double2* post, double* part,
                      unsigned int* counter, double* out_max, unsigned int* err) {
-    const int nrows = c.ny * c.nz;
-    const int grid = xf_div_grid(c.nx / 2, nrows, c.nsm > 0 ? c.nsm : 148);
+    const int grid = xf_div_grid(c.nx / 2, c.ny, c.nz, c.nsm > 0 ? c.nsm : 148, (int)sizeof(V));
     switch (c.nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)c.nx * c.ny * c.nz), k_xf_div<n, V, S>, dim3(grid), dim3(XD<n>::NT), XD<n>::smem, st, mode, c, m, coef, f.ux, f.uy, \
-                   f.uz, spec, twx, post, part, counter, out_max, err); \
+        launch_pdl_if(pdl_pays((size_t)c.nx * c.ny * c.nz), k_xf_div<n, V, S>, dim3(grid), dim3(XD<n>::NT), \
+                      XD<n>::smem(sizeof(V)), st, mode, c, m, coef, f.ux, f.uy, f.uz, spec, twx, post, part, counter, \
+                      out_max, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE

@@ -245,6 +245,13 @@ bool plane_supported(int nx, int nz) {
 #undef P_CASE
     return false;
 }
+size_t plane_smem(int nx, int nz) {
+#define P_CASE(a, b) \
+    if (nx / 2 == a && nz == b) return PK<a, b>::smem;
+    PLANE_PAIRS(P_CASE)
+#undef P_CASE
+    return 0;
+}
 #define PF_TYPES(X, a, b) X(a, b, double, double2)
 #define PB_TYPES(X, a, b) X(a, b, double2, double)
 void plane_init() {
