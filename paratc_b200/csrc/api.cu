@@ -566,13 +566,16 @@ void refresh64(paratc_ctx* ctx) {
     if (ctx->prec == PARATC_PREC_FP32) state_to64(ctx);
 }
 
-int load_state_common(paratc_ctx* ctx, bool wait) {
+// (direct: the FP32 storage form's float arrays hold the new state already)
+int load_state_common(paratc_ctx* ctx, bool wait, bool direct = false) {
     // ChannelInitialize after read_restart (src/m_ChannelSystem.f90:63-68)
     launch_update_uy_ym(ctx->st, ctx->nx * ctx->nz, ctx->d_uy_ym, ctx->d_duy_ym);
     CK(cudaMemcpyAsync(ctx->d_coef, ctx->h_coef0, sizeof(DCoef), cudaMemcpyHostToDevice, ctx->st));
-    launch_bc_all(ctx->st, ctx->kc, ctx->f, ctx->d_uy_ym);
+    const bool s32 = ctx->prec == PARATC_PREC_FP32;
+    if (s32 && direct) launch_bc_all(ctx->st, ctx->kc, ctx->f32, ctx->d_uy_ym);
+    else launch_bc_all(ctx->st, ctx->kc, ctx->f, ctx->d_uy_ym);
     ctx->launches += 2;
-    if (ctx->prec == PARATC_PREC_FP32) state_to32(ctx);
+    if (s32 && !direct) state_to32(ctx);
     return wait ? sync(ctx) : PARATC_OK;
 }
 
@@ -863,12 +866,44 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
     return PARATC_OK;
 }
 
+// whether every non-null array lies in this device's memory, 16-byte aligned
+// (then one kernel moves them all; host arrays go through strided copies)
+static bool on_device(const paratc_ctx* ctx, std::initializer_list<const double*> arrays) {
+    for (const double* a : arrays) {
+        if (!a) continue;
+        cudaPointerAttributes at;
+        if (!aligned16(a) || cudaPointerGetAttributes(&at, a) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeDevice || at.device != ctx->dev) return false;
+    }
+    return true;
+}
+
 static int set_fields_impl(paratc_ctx* ctx, const double* ux, const double* uy, const double* uz, const double* p,
                            const double* c, const double* hx, const double* hy, const double* hz, const double* hc,
                            int layout, bool wait) {
     if (!ctx || (layout != PARATC_LAYOUT_INTERIOR && layout != PARATC_LAYOUT_HALO)) return PARATC_ERR_BAD_ARG;
     CK(cudaSetDevice(ctx->dev));
     ctx->next_ready = false;
+    const bool sc = ctx->prm.scalar_on != 0;
+    if (layout == PARATC_LAYOUT_INTERIOR && ux && uy && uz && p && (c || !sc) &&
+        on_device(ctx, {ux, uy, uz, p, sc ? c : nullptr, hx, hy, hz, sc ? hc : nullptr})) {
+        FieldCopies t{};
+        const bool s32 = ctx->prec == PARATC_PREC_FP32;
+        auto add = [&](double* d, float* d32, const double* h) {
+            t.f[t.n++] = FieldCopies::One{s32 && d32 ? (void*)d32 : (void*)d, const_cast<double*>(h), s32 && d32};
+        };
+        const Fields& f = ctx->f;
+        const Fields32& g = ctx->f32;
+        add(f.ux, g.ux, ux); add(f.uy, g.uy, uy); add(f.uz, g.uz, uz); add(f.pr, nullptr, p);
+        add(f.hx, g.hx, hx); add(f.hy, g.hy, hy); add(f.hz, g.hz, hz);
+        if (sc) { add(f.sc, g.sc, c); add(f.hc, g.hc, hc); }
+        launch_fields(ctx->st, ctx->kc, t, 1);
+        ctx->launches += 1;
+        return load_state_common(ctx, wait, true);
+    }
     struct { double* d; const double* h; bool hist; } tab[] = {
         {ctx->f.ux, ux, false}, {ctx->f.uy, uy, false}, {ctx->f.uz, uz, false}, {ctx->f.pr, p, false},
         {ctx->f.sc, c, false}, {ctx->f.hx, hx, true}, {ctx->f.hy, hy, true}, {ctx->f.hz, hz, true}, {ctx->f.hc, hc, true}};
@@ -899,6 +934,23 @@ static int get_fields_impl(paratc_ctx* ctx, double* ux, double* uy, double* uz, 
                            double* hy, double* hz, double* hc, int layout, bool wait) {
     if (!ctx || (layout != PARATC_LAYOUT_INTERIOR && layout != PARATC_LAYOUT_HALO)) return PARATC_ERR_BAD_ARG;
     CK(cudaSetDevice(ctx->dev));
+    const bool sc = ctx->prm.scalar_on != 0;
+    if (layout == PARATC_LAYOUT_INTERIOR &&
+        on_device(ctx, {ux, uy, uz, p, sc ? c : nullptr, hx, hy, hz, sc ? hc : nullptr})) {
+        FieldCopies t{};
+        const bool s32 = ctx->prec == PARATC_PREC_FP32;
+        auto add = [&](double* d, float* d32, double* h) {
+            if (h) t.f[t.n++] = FieldCopies::One{s32 && d32 ? (void*)d32 : (void*)d, h, s32 && d32};
+        };
+        const Fields& f = ctx->f;
+        const Fields32& g = ctx->f32;
+        add(f.ux, g.ux, ux); add(f.uy, g.uy, uy); add(f.uz, g.uz, uz); add(f.pr, nullptr, p);
+        add(f.hx, g.hx, hx); add(f.hy, g.hy, hy); add(f.hz, g.hz, hz);
+        if (sc) { add(f.sc, g.sc, c); add(f.hc, g.hc, hc); }
+        launch_fields(ctx->st, ctx->kc, t, 0);
+        ctx->launches += t.n > 0;
+        return wait ? sync(ctx) : PARATC_OK;
+    }
     refresh64(ctx);
     struct { double* d; double* h; } tab[] = {{ctx->f.ux, ux}, {ctx->f.uy, uy}, {ctx->f.uz, uz}, {ctx->f.pr, p},
                                              {ctx->f.sc, c}, {ctx->f.hx, hx}, {ctx->f.hy, hy}, {ctx->f.hz, hz}, {ctx->f.hc, hc}};

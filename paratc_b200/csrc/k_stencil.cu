@@ -526,6 +526,41 @@ __global__ void k_cast(size_t n, const A* __restrict__ a, B* __restrict__ b) {
         b[t] = (B)a[t];
 }
 
+// The state between a caller's compact device arrays and the padded fields:
+// every field of a set or get in one launch, a block per stretch of a plane's
+// interior rows (one contiguous run on both sides), pairs of values, four in
+// flight per thread.  Bound by memory.  Replaces a strided copy per field (and,
+// in the FP32 storage form, an FP64 image and a conversion of every array):
+// 1536 x 160 x 256 with scalar, five fields in, four zeroed and nine out, 8.5
+// against 4.3 ms (FP32 storage 10.7 against 2.5 ms).
+constexpr int COPY_U = 4;
+__global__ void __launch_bounds__(256) k_fields(const FieldCopies t, int nx, int ny, int set) {
+    const FieldCopies::One& f = t.f[blockIdx.z];
+    const size_t np = (size_t)ny * nx / 2;  // pairs of a plane's interior rows
+    const size_t q0 = (size_t)blockIdx.x * blockDim.x * COPY_U + threadIdx.x;
+    const size_t po = ((size_t)blockIdx.y * (ny + 2) + 1) * nx / 2;
+    double2* cm = reinterpret_cast<double2*>(f.compact) + (size_t)blockIdx.y * np;
+    double2* p64 = reinterpret_cast<double2*>(f.padded) + po;
+    float2* p32 = reinterpret_cast<float2*>(f.padded) + po;
+    double2 v[COPY_U];
+#pragma unroll
+    for (int u = 0; u < COPY_U; u++) {
+        const size_t q = q0 + (size_t)u * blockDim.x;
+        v[u] = make_double2(0.0, 0.0);
+        if (q >= np) continue;
+        if (!set) v[u] = f.f32 ? make_double2(p32[q].x, p32[q].y) : p64[q];
+        else if (f.compact) v[u] = cm[q];
+    }
+#pragma unroll
+    for (int u = 0; u < COPY_U; u++) {
+        const size_t q = q0 + (size_t)u * blockDim.x;
+        if (q >= np) continue;
+        if (!set) cm[q] = v[u];
+        else if (f.f32) p32[q] = make_float2((float)v[u].x, (float)v[u].y);
+        else p64[q] = v[u];
+    }
+}
+
 // the residual of the discrete pressure Poisson equation r = src - L phi on
 // compact arrays (k*ny + jc-1)*nx + i: L = D4x D4x + D4z D4z + Lyy, the
 // operator whose eigenvalues the spectral solve inverts (D4 the 4th-order
@@ -721,6 +756,13 @@ void launch_cast(cudaStream_t st, size_t n, const double* a, float* b) {
 }
 void launch_cast(cudaStream_t st, size_t n, const float* a, double* b) {
     k_cast<float, double><<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, st>>>(n, a, b);
+}
+
+void launch_fields(cudaStream_t st, const DConst& c, const FieldCopies& t, int set) {
+    const size_t np = (size_t)c.ny * c.nx / 2;
+    if (t.n > 0)
+        k_fields<<<dim3((unsigned)((np + 256 * COPY_U - 1) / (256 * COPY_U)), c.nz, t.n), 256, 0, st>>>(t, c.nx, c.ny,
+                                                                                                         set);
 }
 
 void launch_residual(cudaStream_t st, const DConst& c, const DMetric& m, const double* src, const double* phi,

@@ -85,6 +85,18 @@ void launch_endstep(cudaStream_t st, const DConst& c, const DMetric& m, const Fi
 // storage conversions (FP32 storage form)
 void launch_cast(cudaStream_t st, size_t n, const double* a, float* b);
 void launch_cast(cudaStream_t st, size_t n, const float* a, double* b);
+// fields between compact FP64 device arrays (interior layout, 16-byte aligned)
+// and the padded ones; set with a null compact array writes zeros
+struct FieldCopies {
+    struct One {
+        void* padded;
+        double* compact;
+        int f32;  // the padded field is float
+    };
+    int n;
+    One f[9];
+};
+void launch_fields(cudaStream_t st, const DConst& c, const FieldCopies& t, int set);
 // r = src - L phi (compact arrays) without the pinned kx = kz = 0 equation of
 // row 1, max|r| and max|src| to out[0..1], the row-1 plane means of r and phi
 // to out[2..3]; part holds 4 doubles per cell block
