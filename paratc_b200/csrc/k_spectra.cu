@@ -18,13 +18,13 @@
 // Here two real rows are packed into one complex sequence (a + i b) and
 // transformed with the compile-time-length FFT engine of fft_fixed.cuh; the
 // two real transforms are split off mode by mode (A_k = (Z_k + conj Z_{n-k})/2,
-// B_k = (Z_k - conj Z_{n-k})/2i).  Four packed sequences per row, in the order
-// (ux', ux'_ref), (uy_c, ux_c), (uy, uz), (p, scalar or 0), give every
-// spectrum from one pass over the fields; the ux' modes of the batch stay in
-// shared memory for the cospectrum with uy_c.  A CTA owns one row jc and a
-// contiguous slice of the other direction, B sequences at a time; each thread
-// owns a fixed set of modes and adds its batch sums to the CTA's FP64
-// partial record in a fixed order, and a second kernel adds the slices of a
+// B_k = (Z_k - conj Z_{n-k})/2i).  Four packed sequences per row along z, in
+// the order (ux', ux'_ref), (uy_c, ux_c), (uy, uz), (p, scalar or 0), and three
+// or four along x (see k_spec) give every spectrum from one pass over the
+// fields; the ux' modes of the batch stay in shared memory for the cospectra
+// with uy_c.  A CTA owns one row jc and a contiguous slice of the other
+// direction, B sequences at a time; each thread owns a fixed set of modes and
+// adds its batch sums to the CTA's FP64 partial record in a fixed order, and a second kernel adds the slices of a
 // row in index order, times the norm, to the accumulators.  Results are
 // independent of scheduling.
 #include <algorithm>
@@ -36,7 +36,13 @@
 namespace ptc {
 namespace {
 
-constexpr size_t SPEC_SMEM_BUDGET = 160 * 1024;
+// one record per CTA: NSPEC spectra of NH modes
+constexpr int NSPEC = 9;
+
+// a CTA's shared memory: two CTAs per SM, so that one loads or sums while the
+// other transforms.  Batches as large as that allows, because a batch along z
+// reads B consecutive values of every row (16: whole 128-byte lines)
+constexpr size_t SPEC_SMEM_BUDGET = 110 * 1024;
 
 // launch shape of the length-N spectra kernel: B packed sequences per batch
 // (buffer, ux' modes and twiddles within the shared-memory budget), P threads
@@ -59,10 +65,12 @@ struct SpK {
     }
     static constexpr int P = pcalc();
     static constexpr size_t smem = bytes(B);
+    static constexpr int MINB = smem <= SPEC_SMEM_BUDGET ? 2 : 1;
+    // modes a thread owns (a = tid + q P); their sums stay in registers where
+    // they are few, else in the CTA's record
+    static constexpr int NM = (NH + P - 1) / P;
+    static constexpr bool ACC = NM <= 2;
 };
-
-// one record per CTA: NSPEC spectra of NH modes
-constexpr int NSPEC = 9;
 
 struct SpecTerms {
     // real transforms of the two rows packed in sequence b at mode a
@@ -79,7 +87,7 @@ struct SpecTerms {
 };
 
 template <int N>
-__global__ void __launch_bounds__(SpK<N>::P)
+__global__ void __launch_bounds__(SpK<N>::P, SpK<N>::MINB)
     k_spec(int axis, DConst c, const double* __restrict__ ux, const double* __restrict__ uy,
            const double* __restrict__ uz, const double* __restrict__ pr, const double* __restrict__ sc, int jlcs,
            int splits, const double2* __restrict__ twN, double* __restrict__ part) {
@@ -100,14 +108,25 @@ __global__ void __launch_bounds__(SpK<N>::P)
     const double I1 = c.IC[0], I2 = c.IC[1], I3 = c.IC[2], I4 = c.IC[3], ucrf = c.ucrf;
     const bool has_sc = c.scalar_on != 0;
     double* rec = part + ((size_t)blockIdx.x * splits + s) * NSPEC * NH;
+    constexpr bool ACC = SpK<N>::ACC;
+    constexpr int NM = ACC ? SpK<N>::NM : 1;
+    double acc[NM][NSPEC];
     for (int t = tid; t < N; t += P) tws[t] = twN[t];
-    // a thread zeroes, and later updates, only the modes a = tid + q P of every spectrum
-    for (int a = tid; a < NH; a += P)
-        for (int m = 0; m < NSPEC; m++) rec[m * NH + a] = 0.0;
+#pragma unroll
+    for (int h = 0; h < NM; h++)
+#pragma unroll
+        for (int m = 0; m < NSPEC; m++) acc[h][m] = 0.0;
+    if constexpr (!ACC)
+        for (int a = tid; a < NH; a += P)
+            for (int m = 0; m < NSPEC; m++) rec[m * NH + a] = 0.0;
+    // Along x the cell-centre ux needs no transform of its own: its modes are
+    // those of ux' times the interpolation's transfer function, so three
+    // packed sequences (ux', ux'_ref), (uy_c, p), (uy, uz) do, and (scalar, 0)
+    const int nq = axis == 0 ? (has_sc ? 4 : 3) : 4;
     for (int lb = l0; lb < l1; lb += B) {
         const int nb = min(B, l1 - lb);
 #pragma unroll 1
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < nq; q++) {
             __syncthreads();  // the previous extraction has finished reading buf
             for (int f = tid; f < B * N; f += P) {
                 int b, e;
@@ -121,14 +140,21 @@ __global__ void __launch_bounds__(SpK<N>::P)
                         va = __ldg(&ux[o]) + ucrf;
                         vb = __ldg(&ux[(size_t)k * pl + (size_t)jr * nx + i]) + ucrf;
                     } else if (q == 1) {
-                        const int im = i >= 1 ? i - 1 : nx - 1, ip = i + 1 < nx ? i + 1 : i + 1 - nx;
-                        const int iu = i + 2 < nx ? i + 2 : i + 2 - nx;
-                        const size_t r = o - i;
                         va = 0.5 * (__ldg(&uy[o]) + __ldg(&uy[o + nx]));
-                        vb = I1 * __ldg(&ux[r + im]) + I2 * __ldg(&ux[o]) + I3 * __ldg(&ux[r + ip]) + I4 * __ldg(&ux[r + iu]) + ucrf;
+                        if (axis == 0) {
+                            vb = __ldg(&pr[o]);
+                        } else {
+                            const int im = i >= 1 ? i - 1 : nx - 1, ip = i + 1 < nx ? i + 1 : i + 1 - nx;
+                            const int iu = i + 2 < nx ? i + 2 : i + 2 - nx;
+                            const size_t r = o - i;
+                            vb = I1 * __ldg(&ux[r + im]) + I2 * __ldg(&ux[o]) + I3 * __ldg(&ux[r + ip]) +
+                                 I4 * __ldg(&ux[r + iu]) + ucrf;
+                        }
                     } else if (q == 2) {
                         va = __ldg(&uy[o]);
                         vb = __ldg(&uz[o]);
+                    } else if (axis == 0) {
+                        va = __ldg(&sc[o]);
                     } else {
                         va = __ldg(&pr[o]);
                         vb = has_sc ? __ldg(&sc[o]) : 0.0;
@@ -139,43 +165,68 @@ __global__ void __launch_bounds__(SpK<N>::P)
             __syncthreads();
             ff::smem_passes<N, B, PITCH, P, -1, 0, SC.np>(buf, tws, tid);
             // each thread: its modes a, the batch's sequences in order
-            for (int a = tid; a < NH; a += P) {
+            auto sum_mode = [&](int a, double (&t)[3]) {
                 const int an = a == 0 ? 0 : N - a;
                 const bool edge = (a == 0) || (a == N / 2);
-                double t0 = 0.0, t1 = 0.0, t2 = 0.0;
+                double2 tr = make_double2(0.0, 0.0);  // the interpolation's transfer function at mode a
+                if (axis == 0 && q == 1) {
+                    const double2 w1 = tws[a], w2 = tws[2 * a % N];
+                    tr = make_double2(I1 * w1.x + I2 + I3 * w1.x + I4 * w2.x, I1 * w1.y - I3 * w1.y - I4 * w2.y);
+                }
+                t[0] = t[1] = t[2] = 0.0;
                 for (int b = 0; b < nb; b++) {
                     double2 fa, fb;
                     SpecTerms::split(buf[a * PITCH + b], buf[an * PITCH + b], fa, fb);
                     if (q == 0) {
                         xm[b * NH + a] = fa;
-                        t0 += SpecTerms::energy(fa, edge);
-                        t1 += edge ? fa.x * fb.x : fa.x * fb.x + fa.y * fb.y;
-                        t2 += edge ? 0.0 : fa.y * fb.x - fa.x * fb.y;
+                        t[0] += SpecTerms::energy(fa, edge);
+                        t[1] += edge ? fa.x * fb.x : fa.x * fb.x + fa.y * fb.y;
+                        t[2] += edge ? 0.0 : fa.y * fb.x - fa.x * fb.y;
                     } else if (q == 1) {
-                        t0 += SpecTerms::cosp(xm[b * NH + a], fa, edge);
-                        t1 += SpecTerms::cosp(fb, fa, edge);
+                        const double2 x = xm[b * NH + a];
+                        t[0] += SpecTerms::cosp(x, fa, edge);
+                        t[1] += SpecTerms::cosp(axis == 0 ? cmul(x, tr) : fb, fa, edge);
+                        if (axis == 0) t[2] += SpecTerms::energy(fb, edge);
                     } else {
-                        t0 += SpecTerms::energy(fa, edge);
-                        t1 += SpecTerms::energy(fb, edge);
+                        t[0] += SpecTerms::energy(fa, edge);
+                        t[1] += SpecTerms::energy(fb, edge);
                     }
                 }
-                if (q == 0) {
-                    rec[0 * NH + a] += t0;
-                    rec[6 * NH + a] += t1;
-                    rec[7 * NH + a] += t2;
-                } else if (q == 1) {
-                    rec[4 * NH + a] += t0;
-                    rec[5 * NH + a] += t1;
-                } else if (q == 2) {
-                    rec[1 * NH + a] += t0;
-                    rec[2 * NH + a] += t1;
-                } else {
-                    rec[3 * NH + a] += t0;
-                    rec[8 * NH + a] += t1;
+            };
+            // the spectra that t[0..2] belong to (-1: none)
+            const int m0 = q == 0 ? 0 : q == 1 ? 4 : q == 2 ? 1 : axis == 0 ? 8 : 3;
+            const int m1 = q == 0 ? 6 : q == 1 ? 5 : q == 2 ? 2 : axis == 0 ? -1 : 8;
+            const int m2 = q == 0 ? 7 : q == 1 && axis == 0 ? 3 : -1;
+            if constexpr (ACC) {
+#pragma unroll
+                for (int h = 0; h < NM; h++) {
+                    const int a = tid + h * P;
+                    if (a >= NH) continue;
+                    double t[3];
+                    sum_mode(a, t);
+#pragma unroll
+                    for (int m = 0; m < NSPEC; m++)
+                        acc[h][m] += m == m0 ? t[0] : m == m1 ? t[1] : m == m2 ? t[2] : 0.0;
+                }
+            } else {
+                for (int a = tid; a < NH; a += P) {
+                    double t[3];
+                    sum_mode(a, t);
+                    rec[m0 * NH + a] += t[0];
+                    if (m1 >= 0) rec[m1 * NH + a] += t[1];
+                    if (m2 >= 0) rec[m2 * NH + a] += t[2];
                 }
             }
         }
     }
+    if constexpr (ACC)
+#pragma unroll
+        for (int h = 0; h < NM; h++) {
+            const int a = tid + h * P;
+            if (a < NH)
+#pragma unroll
+                for (int m = 0; m < NSPEC; m++) rec[m * NH + a] = acc[h][m];
+        }
 }
 
 // out[(m*ny + jc-1)*nh + a] += (sum over the row's slices, in order) * norm
@@ -334,7 +385,7 @@ int spectra_splits(const DConst& c, int axis) {
     const int n = axis == 0 ? c.nx : c.nz, nl = axis == 0 ? c.nz : c.nx;
     const int b = spec_batch(n);
     if (b <= 0) return 1;
-    int s = (2 * (c.nsm > 0 ? c.nsm : 148) + c.ny - 1) / c.ny;
+    int s = (6 * (c.nsm > 0 ? c.nsm : 148) + c.ny - 1) / c.ny;  // three waves of CTAs
     const int nbatch = (nl + b - 1) / b;
     if (s > nbatch) s = nbatch;
     return s < 1 ? 1 : s;
