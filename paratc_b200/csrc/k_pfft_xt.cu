@@ -32,7 +32,9 @@
 namespace ptc {
 namespace {
 
-template <int N>
+// VS: bytes of a stored value (8, or 4 for the FP32 storage form's inverse,
+// whose stages hold float2 with the float2 twiddles after them)
+template <int N, int VS = 8>
 struct XT {
     // at least two rows per batch: single-row batches of nx = 3072 ran at 0.40
     // of peak, two-row ones at 0.47 (one CTA per SM)
@@ -51,13 +53,13 @@ struct XT {
     }
     static constexpr int PITCH = pitch();
     static constexpr unsigned STAGE = (unsigned)B * PITCH;  // complex values per stage
-    static constexpr size_t smem = 2 * (size_t)STAGE * sizeof(double2);
+    static constexpr size_t smem = 2 * (size_t)STAGE * 2 * VS + (VS == 4 ? (size_t)N * 8 : 0);
     // resident CTAs that the shared memory allows: the register target of
     // the launch bounds (without it k_xb_tma<1152> takes 236 registers and
     // runs one CTA per SM: 0.28 of peak against 0.39)
     static constexpr int mcalc() {
-        const int m = (int)((220 * 1024) / (smem + 1024));
-        return m < 1 ? 1 : (m > 8 ? 8 : m);
+        const int m = (int)((220 * 1024) / (smem + 1024)), most = VS == 4 ? (768 / P < 1 ? 1 : 768 / P) : 8;
+        return m < 1 ? 1 : (m > most ? most : m);
     }
     static constexpr int MINB = mcalc();
     // between passes the rows are kept in the swizzled order (fft_fixed.cuh):
@@ -195,15 +197,13 @@ __device__ __forceinline__ void xb_tma_body(int nrows, int ny, const Rows& rows,
             tma::bulk_commit();
             const int bn = bt + 2 * gridDim.x;
             if (bn < nb) {
-                tma::bulk_wait_read0();  // the stores have read this stage
+                tma::bulk_wait_read0();  // the lane's stores have read its rows, which it loads next
                 issue(s, bn);
             }
         }
     }
-    if (tid == 0) {
-        tma::bulk_wait0();
-        if (s_bad) xt_fail(mbar, it, nb, err);
-    }
+    if (tid == 0) tma::bulk_wait0();
+    if (tid == 0 && s_bad) xt_fail(mbar, it, nb, err);
 }
 
 template <int N>
@@ -236,16 +236,15 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
 // inputs before a barrier and writes after it; the phi rows leave through
 // coalesced stores of the threads.
 template <int N>
-__global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
+__global__ void __launch_bounds__(XT<N, 4>::P, XT<N, 4>::MINB)
     k_xb_tma32(int nrows, int ny, const float2* __restrict__ spec, float* __restrict__ phi,
                const double2* __restrict__ twN, const double2* __restrict__ post, double scale, int padded,
                unsigned int* __restrict__ err) {
-    constexpr int B = XT<N>::B, P = XT<N>::P, PITCH = XT<N>::PITCH, M1 = N + 1;
+    constexpr int B = XT<N, 4>::B, P = XT<N, 4>::P, PITCH = XT<N, 4>::PITCH, M1 = N + 1;
     static_assert(B % 2 == 0, "row pairs");
     constexpr int NPAIR = B * (N / 2 + 1);
     constexpr int KP = (NPAIR + P - 1) / P;  // merge pairs per thread
-    constexpr unsigned SB = XT<N>::STAGE;
-    static_assert(2 * SB >= (unsigned)N, "the twiddles fit after the float2 stages");
+    constexpr unsigned SB = XT<N, 4>::STAGE;
     constexpr ff::Sched SC = ff::make_sched(N);
     extern __shared__ __align__(128) unsigned char smraw[];
     float2* stage[2] = {reinterpret_cast<float2*>(smraw), reinterpret_cast<float2*>(smraw) + SB};
@@ -268,8 +267,7 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
     pdl_trigger();
     auto issue = [&](int s, int bt) {
         const int g0 = bt * B, nv = min(B, nrows - g0);
-        unsigned bytes = 0;
-        for (int b = 0; b < nv; b += 2) bytes += (unsigned)(b + 1 < nv ? 2 * M1 : M1 + 1) * (unsigned)sizeof(float2);
+        const unsigned bytes = ((unsigned)nv * M1 + (nv & 1)) * (unsigned)sizeof(float2);
         tma::mbar_expect_tx(&mbar[s], bytes);
         for (int b = 0; b < nv; b += 2) {
             const unsigned n2 = (unsigned)(b + 1 < nv ? 2 * M1 : M1 + 1) * (unsigned)sizeof(float2);
@@ -326,7 +324,7 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
             }
         }
         __syncthreads();
-        ff::smem_passes<N, B, PITCH, P, 1, 0, SC.np, 4, true, 0, XT<N>::SWZ>(buf, static_cast<const float2*>(tws),
+        ff::smem_passes<N, B, PITCH, P, 1, 0, SC.np, 4, true, 0, XT<N, 4>::SWZ>(buf, static_cast<const float2*>(tws),
                                                                              tid);
         __syncthreads();
         // phi rows (and the Neumann ghost copies) by coalesced float2 stores
@@ -347,10 +345,8 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
         // the stage's generic reads are done before the next bulk load writes it
         tma::fence_async_smem();
         __syncthreads();
-        if (tid == 0) {
-            const int bn = bt + 2 * gridDim.x;
-            if (bn < nb) issue(s, bn);
-        }
+        const int bn = bt + 2 * gridDim.x;
+        if (tid == 0 && bn < nb) issue(s, bn);
     }
     if (tid == 0 && s_bad) xt_fail(mbar, it, nb, err);
 }
@@ -474,10 +470,8 @@ __device__ __forceinline__ void xf_tma_body(int nrows, const double* __restrict_
             if (tid == 0 && bn < nb) issue(s, bn);
         }
     }
-    if (tid == 0) {
-        tma::bulk_wait0();
-        if (s_bad) xt_fail(mbar, it, nb, err);
-    }
+    if (tid == 0) tma::bulk_wait0();
+    if (tid == 0 && s_bad) xt_fail(mbar, it, nb, err);
 }
 
 template <int N>
@@ -522,7 +516,8 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
 // ---------------------------------------------------------------------------
 constexpr int XD_DIV_U = 2;    // point pairs in flight per producer thread where it does not march (XD::MARCH)
 
-template <int N>
+// VS: bytes of a stored value
+template <int N, int VS>
 struct XD {
     static constexpr int RMAX = ff::Shape<N>::RMAX;
     // rows per batch: the transform's batch, doubled until its thread count
@@ -530,6 +525,9 @@ struct XD {
     static constexpr int bcalc() {
         int b = ff::Shape<N>::B;
         while ((b * N / RMAX) % 32 != 0 && b < 64) b *= 2;
+        // the longer float rows leave the shared memory for twice the
+        // transforming threads
+        if (VS == 4 && N >= 384 && b * N / RMAX < 256) b *= 2;
         return b;
     }
     static constexpr int B = bcalc();
@@ -548,7 +546,7 @@ struct XD {
     // (a multiple or a divisor of the row's pairs, so that none idles)
     static constexpr int Q = !MARCH ? 256
                              : N % 5 == 0 ? 160
-                             : N % 3 == 0 ? (N <= 48 ? 96 : N <= 192 ? 192 : 384)
+                             : N % 3 == 0 ? (N <= 48 ? 96 : N <= 192 ? 192 : 256)
                                           : (N <= 64 ? 128 : 256);
     static constexpr int NT = P + Q;
     // a batch is JB rows jc of KB planes k: row b is plane b / JB, row b % JB
@@ -561,20 +559,19 @@ struct XD {
     static_assert(B % JB == 0, "a batch is whole planes");
     static constexpr int NPT = N >= Q ? (N + Q - 1) / Q : 1;  // pairs per marching thread
     // CTAs per SM: more where the rows are short
-    static constexpr int MINB(int vsize) { return N <= 64 && vsize == 4 ? 3 : (N <= 256 ? 2 : 1); }
-    // shared memory (vsize: bytes of a stored value): the two stages (with
-    // the float2 twiddles after them in the FP32 form), then D planes of the
-    // producers' pairs
-    static constexpr size_t base(int vsize) {
-        return (2 * (size_t)STAGE * 2 * vsize + (vsize == 4 ? (size_t)N * 2 * vsize : 0) + 127) / 128 * 128;
-    }
-    static constexpr size_t plane(int vsize) { return MARCH ? (size_t)NPT * Q * 4 * 2 * vsize : 0; }
-    static constexpr int D(int vsize) {
+    static constexpr int MINB = N <= 64 && VS == 4 ? 3 : (N <= 256 ? 2 : 1);
+    // shared memory: the two stages (with the float2 twiddles after them in the
+    // FP32 form), then D planes of the producers' pairs
+    static constexpr size_t base =
+        (2 * (size_t)STAGE * 2 * VS + (VS == 4 ? (size_t)N * 8 : 0) + 127) / 128 * 128;
+    static constexpr size_t plane = MARCH ? (size_t)NPT * Q * 4 * 2 * VS : 0;
+    static constexpr int dcalc() {
         if (!MARCH) return 0;
-        const int d = (int)(((size_t)(MINB(vsize) == 3 ? 70 : MINB(vsize) == 2 ? 108 : 220) * 1024 - base(vsize)) / plane(vsize));
+        const int d = (int)(((size_t)(MINB == 3 ? 70 : MINB == 2 ? 108 : 220) * 1024 - base) / plane);
         return d < 1 ? 1 : (d > 6 ? 6 : d);
     }
-    static constexpr size_t smem(int vsize) { return base(vsize) + D(vsize) * plane(vsize); }
+    static constexpr int D = dcalc();
+    static constexpr size_t smem = base + D * plane;
 };
 
 // V: storage of the velocity, S: of the spectrum.  The FP32 storage form
@@ -582,28 +579,28 @@ struct XD {
 // stores: a float2 row of N+1 values starts 16-byte aligned only at even
 // rows, which a bulk store needs.
 template <int N, class V, class S>
-__global__ void __launch_bounds__(XD<N>::NT, XD<N>::MINB(sizeof(V)))
+__global__ void __launch_bounds__(XD<N, sizeof(V)>::NT, XD<N, sizeof(V)>::MINB)
     k_xf_div(int mode, DConst c, DMetric m, const DCoef* __restrict__ coef, const V* __restrict__ ux,
              const V* __restrict__ uy, const V* __restrict__ uz, S* __restrict__ spec,
              const double2* __restrict__ twN, const double2* __restrict__ post, double* __restrict__ part,
              unsigned int* __restrict__ counter, double* __restrict__ out_max, unsigned int* __restrict__ err) {
-    constexpr int B = XD<N>::B, P = XD<N>::P, PITCH = XD<N>::PITCH, M1 = N + 1, Q = XD<N>::Q;
+    constexpr int B = XD<N, sizeof(V)>::B, P = XD<N, sizeof(V)>::P, PITCH = XD<N, sizeof(V)>::PITCH, M1 = N + 1, Q = XD<N, sizeof(V)>::Q;
     static_assert(P % 32 == 0, "the consumer group is whole warps");
     // the passes' complex type: float2 for the FP32 storage form (the stages
     // hold float2, half the FP64 stage, and the float2 twiddles sit after
     // them), double2 otherwise (the twiddles read from the global table)
     using A = std::conditional_t<sizeof(S) == sizeof(float2), float2, double2>;
     constexpr bool F32 = sizeof(A) == sizeof(float2);
-    constexpr unsigned SB = XD<N>::STAGE;
+    constexpr unsigned SB = XD<N, sizeof(V)>::STAGE;
     constexpr ff::Sched SC = ff::make_sched(N);
     extern __shared__ __align__(128) unsigned char smraw[];
     A* stage[2] = {reinterpret_cast<A*>(smraw), reinterpret_cast<A*>(smraw) + SB};
     A* tws = stage[0] + 2 * SB;
-    auto* ring = reinterpret_cast<typename MarchPair<V>::T*>(smraw + XD<N>::base(sizeof(V)));
+    auto* ring = reinterpret_cast<typename MarchPair<V>::T*>(smraw + XD<N, sizeof(V)>::base);
     __shared__ unsigned long long full[2], empty[2];
     __shared__ int bad_c, bad_p;
     const int tid = threadIdx.x;
-    constexpr int JB = XD<N>::JB, KB = XD<N>::KB;
+    constexpr int JB = XD<N, sizeof(V)>::JB, KB = XD<N, sizeof(V)>::KB;
     const int ny = c.ny, nz = c.nz;
     // batches in k-fastest order; a CTA takes a contiguous range of them
     const int nbk = (nz + KB - 1) / KB, nb = (ny + JB - 1) / JB * nbk;
@@ -617,7 +614,7 @@ __global__ void __launch_bounds__(XD<N>::NT, XD<N>::MINB(sizeof(V)))
     const long long lim = tma::wait_limit(err);
     const A* tw;
     if constexpr (F32) {
-        for (int t = tid; t < N; t += XD<N>::NT) tws[t] = cto<A>(twN[t]);
+        for (int t = tid; t < N; t += XD<N, sizeof(V)>::NT) tws[t] = cto<A>(twN[t]);
         tw = tws;
     } else {
         tw = reinterpret_cast<const A*>(twN);
@@ -638,7 +635,7 @@ __global__ void __launch_bounds__(XD<N>::NT, XD<N>::MINB(sizeof(V)))
         // producers
         const int tp = tid - P;
         const double sudtal = (mode == 0) ? 1.0 / coef->pmAlpha : 1.0;
-        if constexpr (!XD<N>::MARCH) {
+        if constexpr (!XD<N, sizeof(V)>::MARCH) {
             for (int bt = bt0; bt < bt1; bt++) {
                 const int it = bt - bt0, sg = it & 1, jb = bt / nbk, k = bt - jb * nbk;
                 const bool ok = it < 2 || tma::mbar_wait(&empty[sg], (unsigned)(((it >> 1) + 1) & 1), lim);
@@ -659,7 +656,7 @@ __global__ void __launch_bounds__(XD<N>::NT, XD<N>::MINB(sizeof(V)))
             const int k0 = (bt - jb * nbk) * KB, k1 = min(nz, (be - jb * nbk) * KB);
             const bool mine = jj < JB && jb * JB + jj < ny;
             A* buf = nullptr;
-            const bool ok = div_march<N, Q, XD<N>::NPT, XD<N>::D(sizeof(V))>(
+            const bool ok = div_march<N, Q, XD<N, sizeof(V)>::NPT, XD<N, sizeof(V)>::D>(
                 c, m, ux, uy, uz, jb * JB + jj, e0, mine, k0, k1, sudtal, dm, ring, tp,
                 [&](int k) {
                     if ((k - k0) % KB) return true;
@@ -768,10 +765,10 @@ __global__ void __launch_bounds__(XD<N>::NT, XD<N>::MINB(sizeof(V)))
 #define XT_SIZES(X) X(8) X(12) X(16) X(24) X(32) X(40) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) \
     X(768) X(1024) X(1152) X(1536)
 
-template <int N>
+template <int N, int VS = 8>
 int xt_grid(int nrows, int nsm) {
     const int nb = (nrows + XT<N>::B - 1) / XT<N>::B;
-    const int per_sm = (int)((220 * 1024) / (XT<N>::smem + 1024));
+    const int per_sm = VS == 4 ? XT<N, 4>::MINB : (int)((220 * 1024) / (XT<N>::smem + 1024));
     int grid = (per_sm > 0 ? per_sm : 1) * nsm;
     return grid < nb ? grid : nb;
 }
@@ -791,14 +788,14 @@ bool xt_tma_supported(int n) {
 void xt_tma_init() {
 #define X_CASE(n) \
     cudaFuncSetAttribute(k_xb_tma<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem); \
-    cudaFuncSetAttribute(k_xb_tma32<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem); \
+    cudaFuncSetAttribute(k_xb_tma32<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n, 4>::smem); \
     cudaFuncSetAttribute(k_xf_tma<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem); \
     cudaFuncSetAttribute(k_xb_tma_gather<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);\
     cudaFuncSetAttribute(k_xf_tma_scatter<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XT<n>::smem);\
     cudaFuncSetAttribute(k_xf_div<n, double, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                         (int)XD<n>::smem(8)); \
+                         (int)XD<n, 8>::smem); \
     cudaFuncSetAttribute(k_xf_div<n, float, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                         (int)XD<n>::smem(4));
+                         (int)XD<n, 4>::smem);
     XT_SIZES(X_CASE)
 #undef X_CASE
 }
@@ -824,7 +821,7 @@ void launch_xb_tma(cudaStream_t st, int nx, int ny, int nz, const float2* spec, 
     switch (nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma32<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma32<n>, dim3(xt_grid<n, 4>(nrows, nsm)), dim3(XT<n>::P), XT<n, 4>::smem, st, nrows, ny, \
                    spec, phi, twx, post, scale, padded, err); \
         break;
         XT_SIZES(X_CASE)
@@ -880,12 +877,14 @@ void launch_xf_tma(cudaStream_t st, int nx, int ny, int nz, const double* src, d
 
 // XD::MINB CTAs per SM (the producers' loads and the consumers' transforms
 // share it), at least one batch per CTA
-int xf_div_grid(int n, int ny, int nz, int nsm, int vsize) {
+template <int VS>
+static int xf_div_grid(int n, int ny, int nz, int nsm) {
     switch (n) {
 #define X_CASE(n) \
     case n: { \
-        const int nb = (ny + XD<n>::JB - 1) / XD<n>::JB * ((nz + XD<n>::KB - 1) / XD<n>::KB); \
-        return nb < XD<n>::MINB(vsize) * nsm ? nb : XD<n>::MINB(vsize) * nsm; \
+        using X = XD<n, VS>; \
+        const int nb = (ny + X::JB - 1) / X::JB * ((nz + X::KB - 1) / X::KB); \
+        return nb < X::MINB * nsm ? nb : X::MINB * nsm; \
     }
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -895,7 +894,7 @@ int xf_div_grid(int n, int ny, int nz, int nsm, int vsize) {
 
 bool xf_div_marches(int n) {
     switch (n) {
-#define X_CASE(n) case n: return XD<n>::MARCH;
+#define X_CASE(n) case n: return XD<n, 8>::MARCH;
         XT_SIZES(X_CASE)
 #undef X_CASE
         default: return false;
@@ -906,12 +905,12 @@ template <class V, class S>
 static void xf_div_t(cudaStream_t st, int mode, const DConst& c, const DMetric& m, const DCoef* coef,
                      const FieldSet<V>& f, S* spec, const double2* twx, const double2* post, double* part,
                      unsigned int* counter, double* out_max, unsigned int* err) {
-    const int grid = xf_div_grid(c.nx / 2, c.ny, c.nz, c.nsm > 0 ? c.nsm : 148, (int)sizeof(V));
+    const int grid = xf_div_grid<sizeof(V)>(c.nx / 2, c.ny, c.nz, c.nsm > 0 ? c.nsm : 148);
     switch (c.nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)c.nx * c.ny * c.nz), k_xf_div<n, V, S>, dim3(grid), dim3(XD<n>::NT), \
-                      XD<n>::smem(sizeof(V)), st, mode, c, m, coef, f.ux, f.uy, f.uz, spec, twx, post, part, counter, \
+        launch_pdl_if(pdl_pays((size_t)c.nx * c.ny * c.nz), k_xf_div<n, V, S>, dim3(grid), dim3(XD<n, sizeof(V)>::NT), \
+                      XD<n, sizeof(V)>::smem, st, mode, c, m, coef, f.ux, f.uy, f.uz, spec, twx, post, part, counter, \
                       out_max, err); \
         break;
         XT_SIZES(X_CASE)
