@@ -32,6 +32,14 @@
 namespace ptc {
 namespace {
 
+// lanes of warp 0 that issue the bulk copies of a batch of rows of n complex
+// values, a row each: one thread issuing a batch of short rows in turn cost a
+// small grid several microseconds (inverse of 32 x 24 x 16: 19.3 us by one
+// thread, 12.7 by the lanes; of 128 x 96 x 128 14.8 and 12.8), while a few
+// long rows go out faster from one thread (of 384 x 192 x 256: 98 us, 103 by
+// the lanes; 256 x 256 x 256 is equal)
+constexpr int copy_lanes(int n) { return n <= 64 ? 32 : 1; }
+
 // VS: bytes of a stored value (8, or 4 for the FP32 storage form's inverse,
 // whose stages hold float2 with the float2 twiddles after them)
 template <int N, int VS = 8>
@@ -132,12 +140,14 @@ __device__ __forceinline__ void xb_tma_body(int nrows, int ny, const Rows& rows,
     __syncthreads();
     pdl_wait();  // the spectrum is written by the kernel before this one
     pdl_trigger();
+    constexpr int LN = copy_lanes(N);  // lane l moves rows l, l + LN, ... of a batch, in and out
     auto issue = [&](int s, int bt) {
         const int g0 = bt * B, nv = min(B, nrows - g0);
-        tma::mbar_expect_tx(&mbar[s], (unsigned)nv * M1 * (unsigned)sizeof(double2));
-        for (int b = 0; b < nv; b++) rows.load(stage[s] + b * PITCH, g0 + b, M1, &mbar[s]);
+        if (tid == 0) tma::mbar_expect_tx(&mbar[s], (unsigned)nv * M1 * (unsigned)sizeof(double2));
+        if constexpr (LN > 1) __syncwarp();
+        for (int b = tid; b < nv; b += LN) rows.load(stage[s] + b * PITCH, g0 + b, M1, &mbar[s]);
     };
-    if (tid == 0) {
+    if (tid < LN) {
         if ((int)blockIdx.x < nb) issue(0, blockIdx.x);
         if ((int)(blockIdx.x + gridDim.x) < nb) issue(1, blockIdx.x + gridDim.x);
     }
@@ -178,10 +188,10 @@ __device__ __forceinline__ void xb_tma_body(int nrows, int ny, const Rows& rows,
         ff::smem_passes<N, B, PITCH, P, 1, 0, SC.np, 4, true, 0, XT<N>::SWZ>(buf, twN, tid);
         tma::fence_async_smem();
         __syncthreads();
-        if (tid == 0) {
+        if (tid < LN) {
             const int g0 = bt * B, nv = min(B, nrows - g0);
             constexpr unsigned RB = N * (unsigned)sizeof(double2);
-            for (int b = 0; b < nv; b++) {
+            for (int b = tid; b < nv; b += LN) {
                 const int g = g0 + b;
                 const double2* row = buf + b * PITCH;
                 if (!padded) {
@@ -202,7 +212,7 @@ __device__ __forceinline__ void xb_tma_body(int nrows, int ny, const Rows& rows,
             }
         }
     }
-    if (tid == 0) tma::bulk_wait0();
+    if (tid < LN) tma::bulk_wait0();
     if (tid == 0 && s_bad) xt_fail(mbar, it, nb, err);
 }
 
@@ -265,16 +275,18 @@ __global__ void __launch_bounds__(XT<N, 4>::P, XT<N, 4>::MINB)
     __syncthreads();
     pdl_wait();
     pdl_trigger();
+    constexpr int LN = copy_lanes(N);  // of row pairs
     auto issue = [&](int s, int bt) {
         const int g0 = bt * B, nv = min(B, nrows - g0);
         const unsigned bytes = ((unsigned)nv * M1 + (nv & 1)) * (unsigned)sizeof(float2);
-        tma::mbar_expect_tx(&mbar[s], bytes);
-        for (int b = 0; b < nv; b += 2) {
+        if (tid == 0) tma::mbar_expect_tx(&mbar[s], bytes);
+        if constexpr (LN > 1) __syncwarp();
+        for (int b = 2 * tid; b < nv; b += 2 * LN) {
             const unsigned n2 = (unsigned)(b + 1 < nv ? 2 * M1 : M1 + 1) * (unsigned)sizeof(float2);
             tma::bulk_load(stage[s] + b * M1, spec + (size_t)(g0 + b) * M1, n2, &mbar[s]);
         }
     };
-    if (tid == 0) {
+    if (tid < LN) {
         if ((int)blockIdx.x < nb) issue(0, blockIdx.x);
         if ((int)(blockIdx.x + gridDim.x) < nb) issue(1, blockIdx.x + gridDim.x);
     }
@@ -346,7 +358,7 @@ __global__ void __launch_bounds__(XT<N, 4>::P, XT<N, 4>::MINB)
         tma::fence_async_smem();
         __syncthreads();
         const int bn = bt + 2 * gridDim.x;
-        if (tid == 0 && bn < nb) issue(s, bn);
+        if (tid < LN && bn < nb) issue(s, bn);
     }
     if (tid == 0 && s_bad) xt_fail(mbar, it, nb, err);
 }
@@ -400,13 +412,15 @@ __device__ __forceinline__ void xf_tma_body(int nrows, const double* __restrict_
     __syncthreads();
     pdl_wait();
     pdl_trigger();
+    constexpr int LN = copy_lanes(N);
     auto issue = [&](int s, int bt) {
         const int g0 = bt * B, nv = min(B, nrows - g0);
-        tma::mbar_expect_tx(&mbar[s], (unsigned)nv * N * (unsigned)sizeof(double2));
-        for (int b = 0; b < nv; b++)
+        if (tid == 0) tma::mbar_expect_tx(&mbar[s], (unsigned)nv * N * (unsigned)sizeof(double2));
+        if constexpr (LN > 1) __syncwarp();
+        for (int b = tid; b < nv; b += LN)
             tma::bulk_load(stage[s] + b * PITCH, src + (size_t)(g0 + b) * nx, N * (unsigned)sizeof(double2), &mbar[s]);
     };
-    if (tid == 0) {
+    if (tid < LN) {
         if ((int)blockIdx.x < nb) issue(0, blockIdx.x);
         if ((int)(blockIdx.x + gridDim.x) < nb) issue(1, blockIdx.x + gridDim.x);
     }
@@ -447,9 +461,9 @@ __device__ __forceinline__ void xf_tma_body(int nrows, const double* __restrict_
         if constexpr (Out::bulk) {
             tma::fence_async_smem();
             __syncthreads();
-            if (tid == 0) {
+            if (tid < LN) {
                 const int g0 = bt * B, nv = min(B, nrows - g0);
-                for (int b = 0; b < nv; b++) out.store(g0 + b, buf + b * PITCH, M1);
+                for (int b = tid; b < nv; b += LN) out.store(g0 + b, buf + b * PITCH, M1);
                 tma::bulk_commit();
                 const int bn = bt + 2 * gridDim.x;
                 if (bn < nb) {
@@ -467,10 +481,10 @@ __device__ __forceinline__ void xf_tma_body(int nrows, const double* __restrict_
             tma::fence_async_smem();  // this thread's stage accesses before the refill's async writes
             __syncthreads();          // every thread has read the stage before it is refilled
             const int bn = bt + 2 * gridDim.x;
-            if (tid == 0 && bn < nb) issue(s, bn);
+            if (tid < LN && bn < nb) issue(s, bn);
         }
     }
-    if (tid == 0) tma::bulk_wait0();
+    if (tid < LN) tma::bulk_wait0();
     if (tid == 0 && s_bad) xt_fail(mbar, it, nb, err);
 }
 
@@ -600,6 +614,7 @@ __global__ void __launch_bounds__(XD<N, sizeof(V)>::NT, XD<N, sizeof(V)>::MINB)
     __shared__ unsigned long long full[2], empty[2];
     __shared__ int bad_c, bad_p;
     const int tid = threadIdx.x;
+    [[maybe_unused]] constexpr int LN = copy_lanes(N);
     constexpr int JB = XD<N, sizeof(V)>::JB, KB = XD<N, sizeof(V)>::KB;
     const int ny = c.ny, nz = c.nz;
     // batches in k-fastest order; a CTA takes a contiguous range of them
@@ -737,20 +752,21 @@ __global__ void __launch_bounds__(XD<N, sizeof(V)>::NT, XD<N, sizeof(V)>::MINB)
             }
             tma::fence_async_smem();
             ff::group_sync<1, P>();
-            if (tid == 0) {
-                for (int b = 0; b < B; b++) {
+            if (tid < LN) {
+                for (int b = tid; b < B; b += LN) {
                     const int g = row_of(bt, b);
                     if (g >= 0)
                         tma::bulk_store(reinterpret_cast<double2*>(spec) + (size_t)g * M1, buf + b * PITCH,
                                         M1 * (unsigned)sizeof(double2));
                 }
                 tma::bulk_commit();
-                tma::bulk_wait_read0();  // the stores have read the stage
-                tma::mbar_arrive(&empty[s]);
+                tma::bulk_wait_read0();
+                if constexpr (LN > 1) __syncwarp();  // every lane's stores have read the stage
+                if (tid == 0) tma::mbar_arrive(&empty[s]);
             }
             }
         }
-        if (tid == 0) tma::bulk_wait0();
+        if (tid < LN) tma::bulk_wait0();
     }
     __syncthreads();
     if (tid == 0 && (bad_c | bad_p)) atomicOr(err, 4u);
