@@ -42,7 +42,7 @@ constexpr int NSPEC = 9;
 // a CTA's shared memory: two CTAs per SM, so that one loads or sums while the
 // other transforms.  Batches as large as that allows, because a batch along z
 // reads B consecutive values of every row (16: whole 128-byte lines)
-constexpr size_t SPEC_SMEM_BUDGET = 110 * 1024;
+constexpr size_t SPEC_SMEM_BUDGET = 113 * 1024;
 
 // launch shape of the length-N spectra kernel: B packed sequences per batch
 // (buffer, ux' modes and twiddles within the shared-memory budget), P threads
@@ -53,11 +53,15 @@ struct SpK {
     static constexpr int bcalc() {
         int b = 16;
         while (b > 1 && bytes(b) > SPEC_SMEM_BUDGET) b /= 2;
-        return b;
+        // more butterflies than threads: half the batch and a third CTA (two
+        // butterflies per thread spill; 192 x 96 x 128: 292 -> 256 us,
+        // 256 x 96 x 192: 506 -> 429 us); rows of 512 and more keep the batch
+        // (512 x 96 x 128: 746 against 808 us)
+        return N <= 256 && b * N / RMAX > 256 ? b / 2 : b;
     }
+    static constexpr int RMAX = ff::sched_rmax(N);
     static constexpr int B = bcalc();
     static constexpr int PITCH = B + 1;
-    static constexpr int RMAX = ff::sched_rmax(N);
     static constexpr int pcalc() {
         int p = B * N / RMAX;
         p = (p + 31) / 32 * 32;
@@ -65,7 +69,9 @@ struct SpK {
     }
     static constexpr int P = pcalc();
     static constexpr size_t smem = bytes(B);
-    static constexpr int MINB = smem <= SPEC_SMEM_BUDGET ? 2 : 1;
+    // (three of 192 threads hold 112 registers each without a spill: 96 x 64 x
+    // 96 87 -> 60 us, 768 x 64 x 96 720 -> 618 us)
+    static constexpr int MINB = smem > SPEC_SMEM_BUDGET ? 1 : P == 192 && 3 * (smem + 1024) <= 227 * 1024 ? 3 : 2;
     // modes a thread owns (a = tid + q P); their sums stay in registers where
     // they are few, else in the CTA's record
     static constexpr int NM = (NH + P - 1) / P;
@@ -102,7 +108,9 @@ __global__ void __launch_bounds__(SpK<N>::P, SpK<N>::MINB)
     const int jc = blockIdx.x + 1;
     const int s = blockIdx.y;
     const int nl = axis == 0 ? nz : nx;  // sequences of the row: z planes (x spectra) or x points (z spectra)
-    const int l0 = (int)((long long)nl * s / splits), l1 = (int)((long long)nl * (s + 1) / splits);
+    // a slice is whole batches, so that only the row's last batch is ragged
+    const int nbatch = (nl + B - 1) / B;
+    const int l0 = nbatch * s / splits * B, l1 = min(nl, nbatch * (s + 1) / splits * B);
     const int jr = (c.flow_type == 2 || jc <= ny / 2) ? jlcs : ny + 1 - jlcs;
     const size_t pl = (size_t)c.nyt * nx;
     const double I1 = c.IC[0], I2 = c.IC[1], I3 = c.IC[2], I4 = c.IC[3], ucrf = c.ucrf;
@@ -174,7 +182,9 @@ __global__ void __launch_bounds__(SpK<N>::P, SpK<N>::MINB)
                     tr = make_double2(I1 * w1.x + I2 + I3 * w1.x + I4 * w2.x, I1 * w1.y - I3 * w1.y - I4 * w2.y);
                 }
                 t[0] = t[1] = t[2] = 0.0;
-                for (int b = 0; b < nb; b++) {
+                // (rows past nb are zeros and add nothing)
+#pragma unroll 4
+                for (int b = 0; b < B; b++) {
                     double2 fa, fb;
                     SpecTerms::split(buf[a * PITCH + b], buf[an * PITCH + b], fa, fb);
                     if (q == 0) {
@@ -385,10 +395,10 @@ int spectra_splits(const DConst& c, int axis) {
     const int n = axis == 0 ? c.nx : c.nz, nl = axis == 0 ? c.nz : c.nx;
     const int b = spec_batch(n);
     if (b <= 0) return 1;
-    int s = (6 * (c.nsm > 0 ? c.nsm : 148) + c.ny - 1) / c.ny;  // three waves of CTAs
     const int nbatch = (nl + b - 1) / b;
-    if (s > nbatch) s = nbatch;
-    return s < 1 ? 1 : s;
+    const int s = (6 * (c.nsm > 0 ? c.nsm : 148) + c.ny - 1) / c.ny;  // three waves of CTAs
+    const int per = (nbatch + s - 1) / s;                             // batches of a slice
+    return (nbatch + per - 1) / per;
 }
 
 size_t spectra_part_doubles(const DConst& c) {
