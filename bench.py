@@ -111,7 +111,7 @@ def algorithmic_bytes(params, precision="fp64"):
     wp = 8  # the pressure
     return {
         "rhs": (12 + 4 * sc) * w * N + wp * N,    # u,v,w,p,H* in; Rhs*,H* out
-        "helmholtz": 9 * w * N,                   # Rhs*, u* in; u* out
+        "helmholtz": (9 + 3 * sc) * w * N,        # Rhs*, u* [, c] in; u* [, c] out
         "helmholtz_scalar": 3 * w * N,
         "prsrc": w * (3 * N + S),                 # u,v,w in; x spectrum out (source fused into the x transform)
         "fft_x_fwd": w * (N + S),
