@@ -381,7 +381,7 @@ int paratc_get_precision(paratc_ctx* ctx, int* prec);
  * transforms fed by TMA (persistent CTAs, two shared-memory stages; nz in
  * 128, 256, 512, 768, 1024), 4 as 1 with the divergence source computed by
  * producer warps into the stages of the forward x transform
- * (warp-specialised, one CTA per SM), 5 as 4 with the z transforms of 3;
+ * (warp-specialised), 5 as 4 with the z transforms of 3;
  * y = 0 or 1 (once two kinds of spectral y-solve; one kernel now serves every
  * grid, so both values of y run and time alike).  The x
  * transforms of the separate-transform schedules are fed by bulk copies
