@@ -64,7 +64,9 @@ struct XT {
     static constexpr size_t smem = 2 * (size_t)STAGE * 2 * VS + (VS == 4 ? (size_t)N * 8 : 0);
     // resident CTAs that the shared memory allows: the register target of
     // the launch bounds (without it k_xb_tma<1152> takes 236 registers and
-    // runs one CTA per SM: 0.28 of peak against 0.39)
+    // runs one CTA per SM: 0.28 of peak against 0.39).  The float stages are
+    // half as large, so up to 768 threads share an SM there (1536 x 160 x 256:
+    // 290 -> 269 us)
     static constexpr int mcalc() {
         const int m = (int)((220 * 1024) / (smem + 1024)), most = VS == 4 ? (768 / P < 1 ? 1 : 768 / P) : 8;
         return m < 1 ? 1 : (m > most ? most : m);
@@ -540,7 +542,8 @@ struct XD {
         int b = ff::Shape<N>::B;
         while ((b * N / RMAX) % 32 != 0 && b < 64) b *= 2;
         // the longer float rows leave the shared memory for twice the
-        // transforming threads
+        // transforming threads (with the 256 producers, 1536 x 160 x 256:
+        // 565 -> 473 us)
         if (VS == 4 && N >= 384 && b * N / RMAX < 256) b *= 2;
         return b;
     }

@@ -203,7 +203,7 @@ void launch_xf_tma(cudaStream_t st, int nx, int ny, int nz, const double* src, d
 void launch_xb_tma(cudaStream_t st, int nx, int ny, int nz, const float2* spec, float* phi, const double2* twx,
                    const double2* post, double scale, int padded, int nsm, unsigned int* err);
 // the divergence source of clcPrSrc (mode 0: / pmAlpha, 1: unscaled) and its
-// forward x transform, warp-specialised (one CTA per SM; grid records to part)
+// forward x transform, warp-specialised (at most three CTAs per SM; grid records to part)
 bool xf_div_marches(int n);  // its producers march through k (nx/2 = n)
 void launch_xf_div(cudaStream_t st, int mode, const DConst& c, const DMetric& m, const DCoef* coef, const Fields& f,
                    double2* spec, const double2* twx, const double2* post, double* part, unsigned int* counter,
