@@ -154,8 +154,8 @@ void* paratc_stream(paratc_ctx* ctx);
 
 /* ---- state in / out ---------------------------------------------------- */
 
-/* Loads ux, uy, uz, p (c when scalar_on) and the explicit histories
- * HistX/Y/Z(/C) (NULL = zero), then applies SetBC_and_UpdateHalo,
+/* Loads ux, uy, uz, p (c when scalar_on; NULL keeps the field as it is) and
+ * the explicit histories HistX/Y/Z(/C) (NULL = zero), then applies SetBC_and_UpdateHalo,
  * SetBC_and_UpdateHalo_pr and SetBC_and_UpdateHalo_scalar as
  * ChannelInitialize does (src/m_ChannelSystem.f90:63-68).  ux is the
  * velocity in the computing frame (the restart file holds ux+uCRF). */

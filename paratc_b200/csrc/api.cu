@@ -561,7 +561,7 @@ void state_to64(paratc_ctx* ctx) {
         if (src[q] && dst[q]) { launch_cast(ctx->st, ctx->nf, src[q], dst[q]); ctx->launches++; }
 }
 // before a reader of the FP64 arrays (statistics, spectra, visualisation,
-// restart, get_fields) in the FP32 storage form
+// restart, get_fields) or a partial set_fields in the FP32 storage form
 void refresh64(paratc_ctx* ctx) {
     if (ctx->prec == PARATC_PREC_FP32) state_to64(ctx);
 }
@@ -904,6 +904,9 @@ static int set_fields_impl(paratc_ctx* ctx, const double* ux, const double* uy, 
         ctx->launches += 1;
         return load_state_common(ctx, wait, true);
     }
+    // a state field that is not given keeps its values: in the FP32 storage form
+    // the float arrays hold them, and load_state_common casts the FP64 ones back
+    if (!ux || !uy || !uz || (sc && !c)) refresh64(ctx);
     struct { double* d; const double* h; bool hist; } tab[] = {
         {ctx->f.ux, ux, false}, {ctx->f.uy, uy, false}, {ctx->f.uz, uz, false}, {ctx->f.pr, p, false},
         {ctx->f.sc, c, false}, {ctx->f.hx, hx, true}, {ctx->f.hy, hy, true}, {ctx->f.hz, hz, true}, {ctx->f.hc, hc, true}};

@@ -130,7 +130,7 @@ def test_default_schedule(dims):
 
 
 # state in and out of device arrays: the same bytes as through host arrays, for
-# arrays at any 8-byte address and with some of them left out
+# arrays at any 8-byte address, all of them and half of them read back
 @pytest.mark.parametrize("offset", [0, 1])
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 @pytest.mark.parametrize("dims", [(16, 5, 8), (24, 9, 12), (64, 24, 32)])
@@ -167,6 +167,68 @@ def test_device_state(dims, prec, offset):
             assert np.array_equal(fh[name], fg[name]), name
             if out[i] is not None:
                 assert np.array_equal(out[i].cpu().numpy().reshape(fh[name].shape), fh[name]), name
+
+
+def _dev(a, offset=0):
+    """A device copy of the array, `offset` values past an aligned address."""
+    import torch
+
+    t = torch.zeros(a.size + offset, dtype=torch.float64, device="cuda")[offset:]
+    t.copy_(torch.from_numpy(np.ascontiguousarray(a)).reshape(-1))
+    torch.cuda.synchronize()
+    return t
+
+
+def _address(t):
+    import ctypes
+
+    if t is None:
+        return None
+    return ctypes.cast(t.ctypes.data if isinstance(t, np.ndarray) else t.data_ptr(), ctypes.POINTER(ctypes.c_double))
+
+
+def _device_get(g):
+    """All fields through device arrays."""
+    n = 9 if g.params.scalar_on else 7
+    names = ("ux", "uy", "uz", "p", "c", "hx", "hy", "hz", "hc") if n == 9 else ("ux", "uy", "uz", "p", None, "hx", "hy", "hz", None)
+    t = [_dev(np.zeros(g.shape)) if name else None for name in names]
+    g._check(g._L.paratc_get_fields(g.handle, *[_address(a) for a in t], 0), "get")
+    return {name: a.cpu().numpy().reshape(g.shape) for name, a in zip(names, t) if name}
+
+
+# a state field that a call leaves out keeps its values, whichever way the
+# state before came and the other fields come
+@pytest.mark.parametrize("missing", ["ux", "p", "c"])
+@pytest.mark.parametrize("way", ["host", "device", "unaligned"])
+@pytest.mark.parametrize("before", ["set", "step"])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_field_left_out_is_kept(prec, before, way, missing):
+    case = _half(24, 9, 12)
+    yp = yp_of(case)
+    f = fields_of(case, yp)
+    rng = np.random.default_rng(4)
+    a, b = ([rng.standard_normal((12, 9, 24)) for _ in range(5)] for _ in range(2))
+    with ChannelSystem(case.params, yp) as g:
+        g.set_fields(f["ux"], f["uy"], f["uz"], f["p"], f["c"])
+        g.project()
+        g.precision = prec
+        if before == "set":
+            d = [_dev(x) for x in a] + [None] * 4
+            g._check(g._L.paratc_set_fields(g.handle, *[_address(t) for t in d], 0), "set")
+        else:
+            g.iterate(2, raise_on_guard=False)
+        old = _device_get(g)
+        names = ("ux", "uy", "uz", "p", "c")
+        d = [None if n == missing else x if way == "host" else _dev(x, int(way == "unaligned")) for n, x in zip(names, b)]
+        g._check(g._L.paratc_set_fields(g.handle, *[_address(t) for t in d + [None] * 4], 0), "set")
+        new = g.get_fields()
+        for n, x in zip(names, b):
+            if n == missing:
+                assert np.array_equal(new[n], old[n]), n
+            elif n != "uy":  # (its wall row is the boundary condition's)
+                assert np.array_equal(new[n], x.astype(np.float32) if prec == "fp32" and n != "p" else x), n
+        for n in ("hx", "hy", "hz", "hc"):
+            assert not new[n].any(), n
 
 
 # 1-D spectra: one, two and more modes per thread, rows in one and two batches
