@@ -872,8 +872,9 @@ static bool on_device(const paratc_ctx* ctx, std::initializer_list<const double*
     for (const double* a : arrays) {
         if (!a) continue;
         cudaPointerAttributes at;
-        if (!aligned16(a) || cudaPointerGetAttributes(&at, a) != cudaSuccess) {
-            cudaGetLastError();
+        if (!aligned16(a)) return false;
+        if (cudaPointerGetAttributes(&at, a) != cudaSuccess) {
+            cudaGetLastError();  // this call's own failure: the strided copies report what is wrong
             return false;
         }
         if (at.type != cudaMemoryTypeDevice || at.device != ctx->dev) return false;

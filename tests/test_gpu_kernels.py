@@ -11,7 +11,7 @@ import pytest
 from oracle import oracle_lib as ol
 from paratc_b200 import cases
 from paratc_b200.abi import FT_CH, FT_HC
-from paratc_b200.lib import ChannelSystem
+from paratc_b200.lib import ChannelSystem, ParatcError
 
 from .helpers import fields_of, rel_err, scalar_opts, yp_of
 
@@ -229,6 +229,25 @@ def test_field_left_out_is_kept(prec, before, way, missing):
                 assert np.array_equal(new[n], x.astype(np.float32) if prec == "fp32" and n != "p" else x), n
         for n in ("hx", "hy", "hz", "hc"):
             assert not new[n].any(), n
+
+
+# a CUDA error that an earlier call left is reported by the next sync(),
+# whichever way the arrays of the calls between take
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("call", ["set", "get"])
+def test_pending_error_is_reported(call, offset):
+    import ctypes
+
+    case = _half(16, 5, 8)
+    with ChannelSystem(case.params, yp_of(case)) as g:
+        d = [_dev(np.ones(g.shape), offset) for _ in range(9)]
+        host = np.zeros(8)  # no device memory: the runtime refuses a handle of it
+        assert g._L.paratc_ipc_get_handle(ctypes.c_void_p(host.ctypes.data), ctypes.create_string_buffer(64))
+        f = g._L.paratc_set_fields_async if call == "set" else g._L.paratc_get_fields_async
+        g._check(f(g.handle, *[_address(t) for t in d], 0), call)
+        with pytest.raises(ParatcError):
+            g.sync()
+        g.sync()  # once
 
 
 # 1-D spectra: one, two and more modes per thread, rows in one and two batches
