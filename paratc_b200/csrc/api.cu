@@ -882,6 +882,15 @@ static bool on_device(const paratc_ctx* ctx, std::initializer_list<const double*
     return true;
 }
 
+// whether no two non-null arrays of n values overlap (the strided copies write
+// the fields in their order, one kernel in any)
+static bool disjoint(std::initializer_list<const double*> arrays, size_t n) {
+    for (const double* const* a = arrays.begin(); a != arrays.end(); a++)
+        for (const double* const* b = arrays.begin(); b != a; b++)
+            if (*a && *b && *a < *b + n && *b < *a + n) return false;
+    return true;
+}
+
 static int set_fields_impl(paratc_ctx* ctx, const double* ux, const double* uy, const double* uz, const double* p,
                            const double* c, const double* hx, const double* hy, const double* hz, const double* hc,
                            int layout, bool wait) {
@@ -939,8 +948,8 @@ static int get_fields_impl(paratc_ctx* ctx, double* ux, double* uy, double* uz, 
     if (!ctx || (layout != PARATC_LAYOUT_INTERIOR && layout != PARATC_LAYOUT_HALO)) return PARATC_ERR_BAD_ARG;
     CK(cudaSetDevice(ctx->dev));
     const bool sc = ctx->prm.scalar_on != 0;
-    if (layout == PARATC_LAYOUT_INTERIOR &&
-        on_device(ctx, {ux, uy, uz, p, sc ? c : nullptr, hx, hy, hz, sc ? hc : nullptr})) {
+    const std::initializer_list<const double*> arrays = {ux, uy, uz, p, sc ? c : nullptr, hx, hy, hz, sc ? hc : nullptr};
+    if (layout == PARATC_LAYOUT_INTERIOR && on_device(ctx, arrays) && disjoint(arrays, ctx->ni)) {
         FieldCopies t{};
         const bool s32 = ctx->prec == PARATC_PREC_FP32;
         auto add = [&](double* d, float* d32, double* h) {

@@ -250,6 +250,26 @@ def test_pending_error_is_reported(call, offset):
         g.sync()  # once
 
 
+# arrays of a get that overlap: the fields arrive in their order
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_overlapping_arrays_of_a_get(prec, shift):
+    case = _half(32, 16, 64)
+    rng = np.random.default_rng(5)
+    with ChannelSystem(case.params, yp_of(case)) as g:
+        g.precision = prec
+        g.set_fields(*[rng.standard_normal(g.shape) for _ in range(9)])
+        ref = g.get_fields()
+        n = ref["ux"].size
+        d = _dev(np.zeros(n + 8 * shift * n // 16))
+        t = [d[i * shift * n // 16:] for i in range(9)]
+        expect = np.zeros(d.numel())
+        for i, name in enumerate(g.FIELDS):
+            expect[i * shift * n // 16:][:n] = ref[name].reshape(-1)
+        g._check(g._L.paratc_get_fields(g.handle, *[_address(a) for a in t], 0), "get")
+        assert np.array_equal(d.cpu().numpy(), expect)
+
+
 # 1-D spectra: one, two and more modes per thread, rows in one and two batches
 @pytest.mark.parametrize("dims", [(16, 12, 128), (256, 10, 12), (384, 9, 24), (40, 11, 512), (1536, 5, 30)])
 @pytest.mark.parametrize("make", [_any, _half])
