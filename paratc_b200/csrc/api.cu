@@ -1221,16 +1221,27 @@ extern "C++" {
 //    at 384 x 192 x 256, 1.44 / 1.90 ms at 1536 x 160 x 256.  Rows too long
 //    for the marching producers (nx > 1536) gain in FP64 only (0.97 / 1.27 ms
 //    at 2304 x 64 x 192, 0.79 / 0.67 in the FP32 form).
-//  - z by TMA where nz has the kernel, unless the spectrum's planes are far
-//    apart and short, so that a batch meets a page per row: 1.44 ms with the
-//    register-fed z at 1536 x 160 x 256 (2 MB), 1.55 with TMA.
+//  - z by TMA where nz has the kernel, unless nz <= 256 and the spectrum's
+//    planes are further apart than 3/4 MiB (FP32 form 1/2 MiB), so that a batch
+//    meets a page per row.  Register-fed z against TMA, us per solve, by that
+//    distance.  FP64: 440 / 434 at 384 x 192 x 256 (0.57 MiB), 513 / 512 at 512
+//    x 192 x 256 (0.75), 652 / 673 at 768 x 144 x 256 (0.85), 720 / 756 at 768 x
+//    160 x 256 (0.94), 1442 / 1550 at 1536 x 160 x 256 (1.88); of 24 grids
+//    beyond the line TMA wins by more than 0.4% in one (774 / 765, 768 x 168 x
+//    256).  FP32 form: 412 / 393 at 512 x 192 x 256 (0.38 MiB), 618 / 596 at
+//    768 x 160 x 256 (0.47), 556 / 560 at 512 x 256 x 256 (0.50), 366 / 378 at
+//    1024 x 160 x 128 (0.63), 596 / 631 at 1024 x 256 x 128 (1.00); of 20 grids
+//    beyond the line register-fed z wins by 1.4 to 7% in eight and TMA by 1 to
+//    2.8% in six, among them 1178 / 1152 at 1536 x 160 x 256 (0.94).
 static void default_schedule(paratc_ctx* ctx) {
     const auto off = [](const char* name) { const char* e = std::getenv(name); return e && std::atoi(e) == 0; };
     ctx->plane = ctx->pfft && plane_supported(ctx->nx, ctx->nz) && plane_smem(ctx->nx, ctx->nz) <= 110 * 1024 &&
                  std::getenv("PARATC_NO_PLANE") == nullptr;
-    const size_t apart = (size_t)ctx->ny * ctx->M1 * sizeof(double2);
-    ctx->ztma = ctx->ztma_ok && !ctx->plane && !off("PARATC_ZT_TMA") && !(ctx->nz <= 256 && apart > ((size_t)1 << 20));
-    ctx->xdiv = ctx->xtma && !ctx->plane && (ctx->prec != PARATC_PREC_FP32 || xf_div_marches(ctx->nx / 2));
+    const bool s32 = ctx->prec == PARATC_PREC_FP32;
+    const size_t apart = (size_t)ctx->ny * ctx->M1 * (s32 ? sizeof(float2) : sizeof(double2));
+    const bool far = apart > (size_t)(s32 ? 512 : 768) * 1024;
+    ctx->ztma = ctx->ztma_ok && !ctx->plane && !off("PARATC_ZT_TMA") && !(ctx->nz <= 256 && far);
+    ctx->xdiv = ctx->xtma && !ctx->plane && (!s32 || xf_div_marches(ctx->nx / 2));
 }
 }  // extern "C++"
 

@@ -129,6 +129,21 @@ def test_default_schedule(dims):
             _close(_stepped(case, "fp32"), ref, FP32_VEL, FP32_PR)
 
 
+# the line of the z transform's kind lies at a distance of the spectrum's planes
+# in bytes of the storage form: 3/4 MiB in FP64, 1/2 MiB in the FP32 form
+# (ny (nx / 2 + 1) values of 16 and 8 bytes)
+@pytest.mark.parametrize("dims,fp64,fp32", [((768, 126, 128), 10, 10), ((768, 128, 128), 8, 10), ((768, 170, 128), 8, 10),
+                                            ((768, 172, 128), 8, 8), ((768, 172, 512), 10, 10)])
+def test_default_schedule_line(dims, fp64, fp32):
+    case = _any(*dims)
+    with ChannelSystem(case.params, yp_of(case)) as g:
+        assert g.schedule == fp64
+        g.precision = "fp32"
+        assert g.schedule == fp32
+        g.precision = "fp64"
+        assert g.schedule == fp64
+
+
 # state in and out of device arrays: the same bytes as through host arrays, for
 # arrays at any 8-byte address, all of them and half of them read back
 @pytest.mark.parametrize("offset", [0, 1])
