@@ -112,7 +112,6 @@ def algorithmic_bytes(params, precision="fp64"):
     return {
         "rhs": (12 + 4 * sc) * w * N + wp * N,    # u,v,w,p,H* in; Rhs*,H* out
         "helmholtz": (9 + 3 * sc) * w * N,        # Rhs*, u* [, c] in; u* [, c] out
-        "helmholtz_scalar": 3 * w * N,
         "prsrc": w * (3 * N + S),                 # u,v,w in; x spectrum out (source fused into the x transform)
         "fft_x_fwd": w * (N + S),
         "fft_z_fwd": 2 * w * S,

@@ -34,7 +34,8 @@ bool ptc::pdl_enabled() {
     return on;
 }
 
-// kernel classes of the per-kernel timer
+// kernel classes of the per-kernel timer (PK_HELM_SC keeps its number; the
+// scalar is in PK_HELM's launch)
 enum ProfK {
     PK_COEF = 0, PK_UYYM, PK_RHS, PK_FLOWRATE, PK_HELM, PK_HELM_SC, PK_PRSRC, PK_FFTX_F, PK_FFTZ_F, PK_YSOLVE,
     PK_FFTZ_B, PK_FFTX_B, PK_PROJECT, PK_CFL, PK_CHECK, PK_BC
@@ -70,6 +71,7 @@ struct paratc_ctx {
     bool xtma = false;     // x transforms through the bulk-copy-fed persistent kernels (split path)
     bool xdiv = false;     // the divergence source by producer warps of the forward x transform
     bool sched_auto = true;  // the schedule is default_schedule's, not the caller's
+    int sched_y = 0;         // the y bit of the schedule number: handed back, selects no kernel
     alignas(64) unsigned char zt_tmap[128];  // its tensor map (a CUtensorMap)
     alignas(64) unsigned char zt_tmap32[128];  // the same over the float2 spectrum of the FP32 storage form
     bool ztma32_ok = false;                    // that map is encoded (ncol even, nz supported)
@@ -713,12 +715,6 @@ int paratc_create(const paratc_params* prm, const double* yp, int device, paratc
     kc.nx = ctx->nx; kc.ny = ctx->ny; kc.nz = ctx->nz; kc.nyp = ctx->nyp; kc.nyt = ctx->nyt;
     kc.flow_type = prm->flow_type; kc.scalar_on = prm->scalar_on; kc.is_ux_const = prm->is_ux_const; kc.icfl = prm->icfl;
     cudaDeviceGetAttribute(&kc.nsm, cudaDevAttrMultiProcessorCount, ctx->dev);
-    {
-        // PARATC_YSOLVER=staged|streaming sets the y bit of the schedule
-        // number; every grid takes the same y-solve kernel
-        const char* e = std::getenv("PARATC_YSOLVER");
-        kc.solver_sel = !e ? 0 : (std::strcmp(e, "staged") == 0 ? 1 : (std::strcmp(e, "streaming") == 0 ? 2 : 0));
-    }
     for (int q = 0; q < 4; q++) { kc.dxC[q] = h.dxC[q]; kc.dzC[q] = h.dzC[q]; kc.IC[q] = h.IC[q]; }
     for (int q = 0; q < 5; q++) { kc.dxxC[q] = h.dxxC[q]; kc.dzzC[q] = h.dzzC[q]; }
     kc.rdx = h.rdx; kc.rdz = h.rdz;
@@ -1193,7 +1189,7 @@ int paratc_poisson(paratc_ctx* ctx, const double* src, double* phi) {
     return sync(ctx);
 }
 
-// Poisson schedules: 2*s + (y-1), s 0 fused y-plane transforms, 1 separate
+// Poisson schedules: 2*s + y, s 0 fused y-plane transforms, 1 separate
 // compile-time-length x / z transforms, 2 generic mixed-radix transforms, 3
 // as 1 with TMA-fed z transforms; y, once the kind of the y-solve, selects
 // nothing (one kernel serves every grid) and is only handed back
@@ -1252,14 +1248,14 @@ static void sched_apply(paratc_ctx* ctx, int choice) {
     ctx->pfft = sc == 0 || sc == 1 || sc >= 3;
     ctx->ztma = sc == 3 || sc == 5;
     ctx->xdiv = sc == 4 || sc == 5;
-    ctx->kc.solver_sel = choice % 2 + 1;
+    ctx->sched_y = choice % 2;
     ctx->sched_gen++;
 }
 
 int paratc_get_schedule(paratc_ctx* ctx, int* choice) {
     if (!ctx || !choice) return PARATC_ERR_BAD_ARG;
     const int sc = ctx->plane ? 0 : (ctx->xdiv ? (ctx->ztma ? 5 : 4) : (ctx->ztma ? 3 : (ctx->pfft ? 1 : 2)));
-    *choice = 2 * sc + (ctx->kc.solver_sel == 2 ? 1 : 0);
+    *choice = 2 * sc + ctx->sched_y;
     return PARATC_OK;
 }
 
@@ -2152,10 +2148,10 @@ bool grp_emit(GrpPlan& P, std::map<K, GrpAcc<E>>& m, std::vector<GrpLaunch>& out
 }
 
 // the Poisson schedule of the grouped step: the separate compile-time-length
-// x and z transforms with register-fed z passes (choice 2 or 3, the y-solve
-// kind kept), the form every member of a table shares
+// x and z transforms with register-fed z passes (choice 2 or 3, the y bit
+// kept), the form every member of a table shares
 bool grp_schedule(paratc_ctx* c) {
-    const int y = c->kc.solver_sel == 2 ? 1 : 0;
+    const int y = c->sched_y;
     const bool ok = c->pfft && !c->plane && !c->ztma && !c->xdiv;
     if (ok) return true;
     if (!sched_supported(c, 2 + y)) return false;
@@ -2204,7 +2200,7 @@ int grp_build(paratc_batch* b) {
                                                           the, alp, c->d_part, c->d_counter,
                                                           (int)rhs_member_grid(k, 1).x, 0},
                                        rhs_member_grid(k, 1));
-                h32[k.helm_var].add(k, HelmArgs<float>{k, c->d_coef, c->f32, c->d_duy_ym, c->d_uy_ym, c->d_hfac, 0, k.scalar_on ? 4 : 3},
+                h32[k.helm_var].add(k, HelmArgs<float>{k, c->d_coef, c->f32, c->d_duy_ym, c->d_uy_ym, c->d_hfac, k.scalar_on ? 4 : 3},
                                     helm_member_grid(k, k.scalar_on ? 4 : 3, 4), helm_smem(k, 4));
                 xf32[c->nx].add(k, XfArgs<float, float2>{k, c->dm, c->d_coef, c->f32.ux, c->f32.uy, c->f32.uz, sp,
                                                          c->d_twx, c->d_postx, c->d_part, c->d_counter + 1,
@@ -2225,7 +2221,7 @@ int grp_build(paratc_batch* b) {
                     k, RhsArgs<double>{k, c->dm, c->d_coef, c->f, c->d_uy_ym, c->d_duy_ym, gam, the, alp, c->d_part,
                                        c->d_counter, (int)rhs_member_grid(k, k.fp32_rhs).x, 0},
                     rhs_member_grid(k, k.fp32_rhs));
-                h64[k.helm_var].add(k, HelmArgs<double>{k, c->d_coef, c->f, c->d_duy_ym, c->d_uy_ym, c->d_hfac, 0, k.scalar_on ? 4 : 3},
+                h64[k.helm_var].add(k, HelmArgs<double>{k, c->d_coef, c->f, c->d_duy_ym, c->d_uy_ym, c->d_hfac, k.scalar_on ? 4 : 3},
                                     helm_member_grid(k, k.scalar_on ? 4 : 3, 8), helm_smem(k, 8));
                 xf64[c->nx].add(k, XfArgs<double, double2>{k, c->dm, c->d_coef, c->f.ux, c->f.uy, c->f.uz, sp,
                                                            c->d_twx, c->d_postx, c->d_part, c->d_counter + 1,

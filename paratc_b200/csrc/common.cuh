@@ -40,7 +40,6 @@ struct DConst {
     int nx, ny, nz, nyp, nyt;
     int flow_type, scalar_on, is_ux_const, icfl;
     int nsm;  // streaming multiprocessors of the device
-    int solver_sel;  // the y bit of the schedule number + 1 (0: not set); selects no kernel
     int fp32_rhs;    // 1: the explicit right-hand side computed in FP32 arithmetic (FP64 state)
     int rhs_var;     // compiled launch shape of the FP64 right-hand side (the tuner's pick)
     int helm_var;    // compiled launch shape of the Helmholtz sweeps (the tuner's pick)

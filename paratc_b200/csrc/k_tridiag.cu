@@ -200,8 +200,8 @@ __device__ __forceinline__ void cpa16(void* sdst, const void* gsrc) {
 // are stored in float anyway.  G: the block this CTA works as (OwnGrid, or
 // SubGrid in a grouped launch).
 template <class V, int U, class W, class G>
-__device__ __forceinline__ void helm_body(const G& grid, const DConst& cst, const DCoef* __restrict__ coef, int comp0,
-                                          int ncomp, const FieldSet<V>& fl, const double* __restrict__ duy_ym,
+__device__ __forceinline__ void helm_body(const G& grid, const DConst& cst, const DCoef* __restrict__ coef, int ncomp,
+                                          const FieldSet<V>& fl, const double* __restrict__ duy_ym,
                                           const double* __restrict__ uy_ym, const double* __restrict__ facs) {
     using WP = typename W2<W>::T;
     constexpr int VL = 16 / (int)sizeof(V), LPR = 32 / VL, RPW = 32 / LPR;  // a copy's columns, lanes per row, rows per pass
@@ -230,7 +230,7 @@ __device__ __forceinline__ void helm_body(const G& grid, const DConst& cst, cons
         const int c = item / nct, q = (item - c * nct) * 32 + lc;
         cval = q < ncols;
         const int k = q / nx;
-        csrc = rhs_of(comp0 + c) + (size_t)k * pl + (q - k * nx) + (size_t)jw * nx + lr * gstep;
+        csrc = rhs_of(c) + (size_t)k * pl + (q - k * nx) + (size_t)jw * nx + lr * gstep;
     };
     auto copy_rows = [&](int i0, int n) {  // rows i0 .. i0 + n - 1, n <= U
         const V* src = csrc + i0 * gstep;
@@ -250,7 +250,7 @@ __device__ __forceinline__ void helm_body(const G& grid, const DConst& cst, cons
     for (int it = 0; item < nitems; item += stride, it++) {
         const int next = item + stride;
         if (next >= nitems) pdl_trigger();
-        const int comp = comp0 + item / nct;
+        const int comp = item / nct;
         const int t = comp == 1 ? 1 : (comp == 3 ? 2 : 0);
         if (t != type) {  // this matrix's table, in sweep order
             type = t;
@@ -373,17 +373,17 @@ __device__ __forceinline__ void helm_body(const G& grid, const DConst& cst, cons
 }
 
 template <class V, int U, class W = double>
-__global__ void __launch_bounds__(64, 8) k_helm(DConst cst, const DCoef* __restrict__ coef, int comp0, int ncomp,
-                                                FieldSet<V> fl, const double* __restrict__ duy_ym,
+__global__ void __launch_bounds__(64, 8) k_helm(DConst cst, const DCoef* __restrict__ coef, int ncomp, FieldSet<V> fl,
+                                                const double* __restrict__ duy_ym,
                                                 const double* __restrict__ uy_ym, const double* __restrict__ facs) {
-    helm_body<V, U, W>(OwnGrid{}, cst, coef, comp0, ncomp, fl, duy_ym, uy_ym, facs);
+    helm_body<V, U, W>(OwnGrid{}, cst, coef, ncomp, fl, duy_ym, uy_ym, facs);
 }
 
 template <class V, int U, class W = double>
 __global__ void __launch_bounds__(64, 8) k_helm_grp(const GrpTab<HelmArgs<V>>* __restrict__ t) {
     SubGrid g;
     const HelmArgs<V>& a = t->e[grp_member(t, g)];
-    helm_body<V, U, W>(g, a.c, a.coef, a.comp0, a.ncomp, a.fl, a.duy_ym, a.uy_ym, a.fac);
+    helm_body<V, U, W>(g, a.c, a.coef, a.ncomp, a.fl, a.duy_ym, a.uy_ym, a.fac);
 }
 
 // ---------------------------------------------------------------------------
@@ -826,26 +826,27 @@ void launch_helm_grp(cudaStream_t st, const DConst& key, const GrpTab<HelmArgs<f
 }
 
 template <class V>
-static void helm_dispatch(cudaStream_t st, const DConst& c, const DCoef* coef, int comp0, int ncomp,
-                          const FieldSet<V>& f, const double* duy_ym, const double* uy_ym, const double* fac) {
+static void helm_dispatch(cudaStream_t st, const DConst& c, const DCoef* coef, const FieldSet<V>& f,
+                          const double* duy_ym, const double* uy_ym, const double* fac) {
     using WF = std::conditional_t<sizeof(V) == 4, float, double>;
+    const int ncomp = c.scalar_on ? 4 : 3;
     const dim3 g = helm_member_grid(c, ncomp, sizeof(V)), b(64);
     const size_t smem = helm_smem(c, sizeof(V));
     if (c.helm_var == 1)
-        launch_pdl(k_helm<V, HY_U / 2>, g, b, smem, st, c, coef, comp0, ncomp, f, duy_ym, uy_ym, fac);
+        launch_pdl(k_helm<V, HY_U / 2>, g, b, smem, st, c, coef, ncomp, f, duy_ym, uy_ym, fac);
     else if (helm_float(c, sizeof(V)))
-        launch_pdl(k_helm<V, HY_U, WF>, g, b, smem, st, c, coef, comp0, ncomp, f, duy_ym, uy_ym, fac);
+        launch_pdl(k_helm<V, HY_U, WF>, g, b, smem, st, c, coef, ncomp, f, duy_ym, uy_ym, fac);
     else
-        launch_pdl(k_helm<V, HY_U>, g, b, smem, st, c, coef, comp0, ncomp, f, duy_ym, uy_ym, fac);
+        launch_pdl(k_helm<V, HY_U>, g, b, smem, st, c, coef, ncomp, f, duy_ym, uy_ym, fac);
 }
 
 void launch_helm(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields& f, const double* duy_ym,
                  const double* uy_ym, const double* fac) {
-    helm_dispatch(st, c, coef, 0, c.scalar_on ? 4 : 3, f, duy_ym, uy_ym, fac);
+    helm_dispatch(st, c, coef, f, duy_ym, uy_ym, fac);
 }
 void launch_helm(cudaStream_t st, const DConst& c, const DCoef* coef, const Fields32& f, const double* duy_ym,
                  const double* uy_ym, const double* fac) {
-    helm_dispatch(st, c, coef, 0, c.scalar_on ? 4 : 3, f, duy_ym, uy_ym, fac);
+    helm_dispatch(st, c, coef, f, duy_ym, uy_ym, fac);
 }
 
 void launch_ysolve(cudaStream_t st, const DConst& c, const DMetric& m, double2* spec) {

@@ -282,12 +282,12 @@ struct RhsArgs {  // k_rhs_tile
     int pad;
 };
 template <class V>
-struct HelmArgs {  // k_helm, components comp0 .. comp0 + ncomp - 1
+struct HelmArgs {  // k_helm, components 0 .. ncomp - 1
     DConst c;
     const DCoef* coef;
     FieldSet<V> fl;
     const double *duy_ym, *uy_ym, *fac;
-    int comp0, ncomp;
+    int ncomp;
 };
 template <class V, class S>
 struct XfArgs {  // k_xf, divergence source of the substep (mode 0)
