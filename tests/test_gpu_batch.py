@@ -116,7 +116,7 @@ def test_batch_recaptures_after_schedule_change():
         s.iterate(3)
     _same(b, singles)
     for g in (b.members[1], singles[1]):
-        g.schedule = 5  # generic transforms, streaming y-solve
+        g.schedule = 5  # generic transforms, y bit set
     b.iterate(3, use_graph=True)
     for s in singles:
         s.iterate(3)

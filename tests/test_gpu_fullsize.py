@@ -1,7 +1,7 @@
 """Parity at the benchmark sizes themselves.
 
-C2 (512 x 256 x 512) reaches the kernels only large grids use (the streaming
-y-solve, 512-point z transforms, 256-point x transforms); the oracle solves
+C2 (512 x 256 x 512) reaches the kernels only large grids use (the
+512-point z transforms, 256-point x transforms); the oracle solves
 it in a few seconds on the host.  C1 (128 x 96 x 128) is the bench workload:
 two full RK3 steps against the oracle, the solenoidality of the result, and
 the 1-D spectra of the stepped fields; then its stated horizon, 100 RK3

@@ -1,12 +1,10 @@
 """Parity of the alternative kernel variants that size selects automatically.
 
-The spectral y-solve has a staged variant (whole column strips copied to
-shared memory first) and a streaming variant (rows streamed from HBM), chosen
-by grid size; the Poisson transforms have compile-time-length kernels and a
-generic Stockham path for lengths outside their list.  The small grids of
-the other tests reach only one variant of each, so here every variant is
-forced through the environment (read when a context is created) and
-compared with the oracle.  Tolerances as in test_gpu_parity.
+The Poisson transforms have one-CTA-per-plane kernels, compile-time-length
+kernels and a generic Stockham path for lengths outside their list.  The small
+grids of the other tests reach only some of them, so here every variant is
+forced through the schedule or the environment (read when a context is
+created) and compared with the oracle.  Tolerances as in test_gpu_parity.
 """
 import pytest
 
@@ -24,11 +22,13 @@ TOL_STEPS = 1e-8
 TOL_POISSON = 1e-12
 
 
-def _steps_vs_oracle(case, nsteps):
+def _steps_vs_oracle(case, nsteps, schedule=None):
     yp = yp_of(case)
     f = fields_of(case, yp)
     o = ol.Oracle(case.params, yp)
     g = ChannelSystem(case.params, yp)
+    if schedule is not None:
+        g.schedule = schedule
     o.set_fields(f["ux"], f["uy"], f["uz"], f["p"], f["c"])
     g.set_fields(f["ux"], f["uy"], f["uz"], f["p"], f["c"])
     for s in range(nsteps):
@@ -44,19 +44,30 @@ def _steps_vs_oracle(case, nsteps):
             assert e <= tol, "%s step %d: %s rel err %.3e" % (case.name, s + 1, n, e)
 
 
-@pytest.mark.parametrize("solver", ["staged", "streaming"])
 @pytest.mark.parametrize("name", ["channel", "halfchannel_scalar"])
-def test_solver_variants_steps(monkeypatch, solver, name):
-    monkeypatch.setenv("PARATC_YSOLVER", solver)
-    _steps_vs_oracle(variant(name), 3)
+def test_solver_variants_steps(name):
+    """The y bit of the schedule number is handed back and changes no result."""
+    case = variant(name)
+    yp = yp_of(case)
+    f = fields_of(case, yp)
+    out = []
+    for y in (0, 1):
+        with ChannelSystem(case.params, yp) as g:
+            g.schedule = 2 + y
+            assert g.schedule == 2 + y
+            g.set_fields(f["ux"], f["uy"], f["uz"], f["p"], f["c"])
+            g.iterate(2, raise_on_guard=False)
+            out.append(g.get_fields())
+    for n in out[0]:
+        assert (out[0][n] == out[1][n]).all(), n
+    _steps_vs_oracle(case, 3, schedule=3)
 
 
-@pytest.mark.parametrize("solver", [None, "staged", "streaming"])
-def test_tall_columns(monkeypatch, solver):
-    """A tall grid (ny = 120): long dependent chains in every y-solve."""
-    if solver:
-        monkeypatch.setenv("PARATC_YSOLVER", solver)
-    _steps_vs_oracle(cases.small_channel(16, 120, 8), 2)
+@pytest.mark.parametrize("ny", [120, 122, 254, 256])
+def test_tall_columns(ny):
+    """Tall grids, up to the tallest: long dependent chains in every y-solve,
+    with and without a remainder of the rows a sweep reads ahead."""
+    _steps_vs_oracle(cases.small_channel(16, ny, 8), 2)
 
 
 @pytest.mark.parametrize("dims", [(24, 20, 30), (32, 24, 16)])
@@ -88,15 +99,19 @@ def test_fixed_length_sizes(dims):
 @pytest.mark.parametrize("dims", [(64, 24, 64), (96, 20, 96), (128, 96, 128)])
 def test_plane_and_split_transforms(monkeypatch, plane, dims):
     """The one-CTA-per-plane transforms (k_plane.cu) and the separate x / z
-    kernels on the same grids (plane pairs (32,64), (48,96), (64,128))."""
+    kernels on the same grids (plane pairs (32,64), (48,96), (64,128)); the
+    largest planes are not the default's choice."""
     if not plane:
         monkeypatch.setenv("PARATC_NO_PLANE", "1")
     case = cases.small_channel(*dims)
     yp = yp_of(case)
     src = cases.gaussian_source(cases.Case("src", case.params, case.mesh, "gauss_src", 11, 1.0))
     phi_o = ol.Oracle(case.params, yp).poisson(src)
-    phi_g = ChannelSystem(case.params, yp).poisson(src)
-    assert rel_err(phi_g, phi_o) <= TOL_POISSON
+    g = ChannelSystem(case.params, yp)
+    assert (g.schedule == 0) == (plane and dims[0] < 128)
+    if plane:
+        g.schedule = 0
+    assert rel_err(g.poisson(src), phi_o) <= TOL_POISSON
     if dims[1] <= 24:
         _steps_vs_oracle(case, 2)
 
@@ -106,8 +121,7 @@ def test_schedules_and_autotune(dims):
     """Every Poisson schedule this grid supports (fused plane transforms,
     separate fixed-length transforms, generic transforms, separate transforms
     with TMA-fed z passes, the same with the warp-specialised divergence
-    source of the x transform; staged or streaming y-solve) gives the oracle's
-    fields after two steps; the auto-tuner times all of them and keeps the
+    source of the x transform) gives the oracle's fields after two steps; the auto-tuner times all of them and keeps the
     fastest."""
     case = cases.small_channel(*dims)
     yp = yp_of(case)
