@@ -1213,10 +1213,12 @@ extern "C++" {
 //    fused against separate: 37 / 49 us per solve of 96 x 96 x 96, 33 / 44 of
 //    64 x 96 x 128, 53 / 50 of 128 x 96 x 128.
 //  - Else the divergence by the producers of the forward x transform, against
-//    computing it in the transform: 73 / 90 us at 192 x 96 x 128, 459 / 518
+//    computing it in the transform: 73 / 90 us at 192 x 96 x 128, 440 / 523
 //    at 384 x 192 x 256, 1.44 / 1.90 ms at 1536 x 160 x 256.  Rows too long
 //    for the marching producers (nx > 1536) gain in FP64 only (0.97 / 1.27 ms
-//    at 2304 x 64 x 192, 0.79 / 0.67 in the FP32 form).
+//    at 2304 x 64 x 192, 0.79 / 0.67 in the FP32 form).  FP32 form: 343 / 385
+//    at 384 x 192 x 256; of 18 smaller grids' steps 13 are shorter by 1 to 15%,
+//    four equal within 1% and one longer (520 / 492 us, 96 x 96 x 192).
 //  - z by TMA where nz has the kernel, unless nz <= 256 and the spectrum's
 //    planes are further apart than 3/4 MiB (FP32 form 1/2 MiB), so that a batch
 //    meets a page per row.  Register-fed z against TMA, us per solve, by that

@@ -305,9 +305,9 @@ static void pfft_xf_t(cudaStream_t st, int mode, const DConst& c, const DMetric&
     switch (c.nx / 2) {
 #define X_CASE(n)                                                                                              \
     case n:                                                                                                    \
-        launch_pdl_if(pdl_pays((size_t)nrows * 2 * n), k_xf<n, V, S, A>, dim3((nrows + XK<n, A>::B - 1) / XK<n, A>::B), dim3(XK<n, A>::P),        \
-                   XK<n, A>::smem, st, mode, c, m, coef, f.ux, f.uy, f.uz, src, spec, twx, post, part, counter,  \
-                   out_max);                                                                                   \
+        launch_pdl_if(pdl_pays((size_t)nrows * 2 * n), k_xf<n, V, S, A>, \
+                      dim3((nrows + XK<n, A>::B - 1) / XK<n, A>::B), dim3(XK<n, A>::P), XK<n, A>::smem, st, mode, \
+                      c, m, coef, f.ux, f.uy, f.uz, src, spec, twx, post, part, counter, out_max); \
         break;
         PFFT_X_SIZES(X_CASE)
 #undef X_CASE
@@ -324,8 +324,9 @@ static void pfft_xb_t(cudaStream_t st, int nx, int ny, int nz, const S* spec, PH
     switch (nx / 2) {
 #define X_CASE(n)                                                                                              \
     case n:                                                                                                    \
-        launch_pdl_if(pdl_pays((size_t)nrows * 2 * n), k_xb<n, S, PH, A>, dim3((nrows + XK<n, A>::B - 1) / XK<n, A>::B), dim3(XK<n, A>::P),      \
-                   XK<n, A>::smem, st, ny, nz, spec, phi, twx, post, scale, padded, accumulate, shift);        \
+        launch_pdl_if(pdl_pays((size_t)nrows * 2 * n), k_xb<n, S, PH, A>, \
+                      dim3((nrows + XK<n, A>::B - 1) / XK<n, A>::B), dim3(XK<n, A>::P), XK<n, A>::smem, st, ny, \
+                      nz, spec, phi, twx, post, scale, padded, accumulate, shift); \
         break;
         PFFT_X_SIZES(X_CASE)
 #undef X_CASE

@@ -525,10 +525,10 @@ __global__ void __launch_bounds__(XT<N>::P, XT<N>::MINB)
 // planes of JB rows and a CTA takes a contiguous range of batches in k-fastest
 // order.  The transform by the same threads that compute the divergence (k_xf)
 // waits for nine loads per pair of points with few of them in flight.  One
-// B200, divergence and transform, k_xf against this kernel: 258 / 172 us at
-// 384 x 192 x 256, 1.06 / 0.63 ms at 1536 x 160 x 256 (0.31 ms of memory at
+// B200, divergence and transform, k_xf against this kernel: 255 / 171 us at
+// 384 x 192 x 256, 1.05 / 0.63 ms at 1536 x 160 x 256 (0.31 ms of memory at
 // the copy rate; there the 192 transforming threads of an SM set the pace),
-// 28 / 27 us at 128 x 96 x 128.
+// 25 / 27 us at 128 x 96 x 128, whose solve is shorter all the same (56 / 50).
 // ---------------------------------------------------------------------------
 constexpr int XD_DIV_U = 2;    // point pairs in flight per producer thread where it does not march (XD::MARCH)
 
@@ -601,7 +601,8 @@ __global__ void __launch_bounds__(XD<N, sizeof(V)>::NT, XD<N, sizeof(V)>::MINB)
              const V* __restrict__ uy, const V* __restrict__ uz, S* __restrict__ spec,
              const double2* __restrict__ twN, const double2* __restrict__ post, double* __restrict__ part,
              unsigned int* __restrict__ counter, double* __restrict__ out_max, unsigned int* __restrict__ err) {
-    constexpr int B = XD<N, sizeof(V)>::B, P = XD<N, sizeof(V)>::P, PITCH = XD<N, sizeof(V)>::PITCH, M1 = N + 1, Q = XD<N, sizeof(V)>::Q;
+    constexpr int B = XD<N, sizeof(V)>::B, P = XD<N, sizeof(V)>::P, Q = XD<N, sizeof(V)>::Q;
+    constexpr int PITCH = XD<N, sizeof(V)>::PITCH, M1 = N + 1;
     static_assert(P % 32 == 0, "the consumer group is whole warps");
     // the passes' complex type: float2 for the FP32 storage form (the stages
     // hold float2, half the FP64 stage, and the float2 twiddles sit after
@@ -825,8 +826,8 @@ void launch_xb_tma(cudaStream_t st, int nx, int ny, int nz, const double2* spec,
     switch (nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, spec, \
-                   phi, twx, post, scale, padded, err); \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), \
+                      XT<n>::smem, st, nrows, ny, spec, phi, twx, post, scale, padded, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -840,8 +841,8 @@ void launch_xb_tma(cudaStream_t st, int nx, int ny, int nz, const float2* spec, 
     switch (nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma32<n>, dim3(xt_grid<n, 4>(nrows, nsm)), dim3(XT<n>::P), XT<n, 4>::smem, st, nrows, ny, \
-                   spec, phi, twx, post, scale, padded, err); \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma32<n>, dim3(xt_grid<n, 4>(nrows, nsm)), dim3(XT<n>::P), \
+                      XT<n, 4>::smem, st, nrows, ny, spec, phi, twx, post, scale, padded, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -855,8 +856,8 @@ void launch_xb_tma_gather(cudaStream_t st, int nx, int ny, int nz, const XtGathe
     switch (nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma_gather<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, ny, \
-                   gt, phi, twx, post, scale, err); \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xb_tma_gather<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), \
+                      XT<n>::smem, st, nrows, ny, gt, phi, twx, post, scale, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -870,8 +871,8 @@ void launch_xf_tma_scatter(cudaStream_t st, int nx, int ny, int nz, const double
     switch (nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xf_tma_scatter<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, \
-                   ny, src, gt, twx, post, err); \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xf_tma_scatter<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), \
+                      XT<n>::smem, st, nrows, ny, src, gt, twx, post, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE
@@ -885,8 +886,8 @@ void launch_xf_tma(cudaStream_t st, int nx, int ny, int nz, const double* src, d
     switch (nx / 2) {
 #define X_CASE(n) \
     case n: \
-        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xf_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), XT<n>::smem, st, nrows, src, spec, \
-                   twx, post, err); \
+        launch_pdl_if(pdl_pays((size_t)nrows * nx), k_xf_tma<n>, dim3(xt_grid<n>(nrows, nsm)), dim3(XT<n>::P), \
+                      XT<n>::smem, st, nrows, src, spec, twx, post, err); \
         break;
         XT_SIZES(X_CASE)
 #undef X_CASE

@@ -160,9 +160,10 @@ static void pfft_z_t(cudaStream_t st, int dir, int nx, int ny, int nz, S* spec, 
 #define Z_CASE(n)                                                                                                 \
     case n: {                                                                                                     \
         const int grid = (ncol + ZK<n, A>::B - 1) / ZK<n, A>::B;                                                  \
-        if (dir < 0)                                                                                              \
-            launch_pdl_if(pdl_pays((size_t)2 * ncol * n), k_zt<n, -1, S, A>, dim3(grid), dim3(ZK<n, A>::P), ZK<n, A>::smem, st, ncol, spec, twz);    \
-        else launch_pdl_if(pdl_pays((size_t)2 * ncol * n), k_zt<n, 1, S, A>, dim3(grid), dim3(ZK<n, A>::P), ZK<n, A>::smem, st, ncol, spec, twz);    \
+        const bool early = pdl_pays((size_t)2 * ncol * n);                                                        \
+        const dim3 grd(grid), blk(ZK<n, A>::P);                                                                   \
+        if (dir < 0) launch_pdl_if(early, k_zt<n, -1, S, A>, grd, blk, ZK<n, A>::smem, st, ncol, spec, twz);      \
+        else launch_pdl_if(early, k_zt<n, 1, S, A>, grd, blk, ZK<n, A>::smem, st, ncol, spec, twz);               \
         break;                                                                                                    \
     }
         PFFT_Z_SIZES(Z_CASE)

@@ -398,7 +398,7 @@ int spectra_splits(const DConst& c, int axis) {
     const int b = spec_batch(n);
     if (b <= 0) return 1;
     const int nbatch = (nl + b - 1) / b;
-    const int s = (6 * (c.nsm > 0 ? c.nsm : 148) + c.ny - 1) / c.ny;  // three waves of CTAs
+    const int s = (6 * (c.nsm > 0 ? c.nsm : 148) + c.ny - 1) / c.ny;  // three waves of CTAs, two where three share an SM (MINB)
     const int per = (nbatch + s - 1) / s;                             // batches of a slice
     return (nbatch + per - 1) / per;
 }
